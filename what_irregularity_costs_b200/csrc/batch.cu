@@ -173,7 +173,7 @@ public:
             // one-time host query has happened), then replayed.
             if (!have) {
                 drop_graph();
-                if ((e = capture(w, shape)) != cudaSuccess) return e;
+                if ((e = capture(w, shape)) != cudaSuccess) return e;  // nothing ran
             }
             e = cudaGraphLaunch(exec_, stream_);
         } else {
@@ -181,6 +181,9 @@ public:
             ran_n_ = n;
             ran_shape_ = shape;
         }
+        if (e != cudaSuccess)  // some passes may have run without the others
+            for (Volume* v : vols_)
+                if (v) v->mark_unfinished();
         if (tuning_) {
             cudaEventRecord(t1, stream_);
             tune_log_.push_back(TuneStep{tune_index_, t0, t1});

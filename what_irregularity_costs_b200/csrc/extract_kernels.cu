@@ -24,6 +24,7 @@ namespace osn_b200 {
 namespace {
 
 constexpr int kExtractThreads = 512;
+constexpr int kResetThreads = 128;
 constexpr int kHalo = 9;
 constexpr int kHaloCells = kHalo * kHalo * kHalo;
 
@@ -439,43 +440,37 @@ __global__ void list_blocks_kernel(const HashEntry* table, uint32_t size, int32_
     }
 }
 
-// Zero the voxels of the blocks of a list, one CTA per block.
-__global__ void reset_listed_kernel(DevVolume v, const int32_t* list, int32_t n) {
-    const int32_t i = blockIdx.x;
-    if (i >= n) return;
-    const size_t b = (size_t)list[i];
-    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-    const int n_t = kBlockVoxels * tsdf_bytes(v.storage) / 16;
-    const int n_w = kBlockVoxels * weight_bytes(v.storage) / 16;
-    for (int k = threadIdx.x; k < n_t; k += blockDim.x) {
-        reinterpret_cast<float4*>(v.tsdf)[b * n_t + k] = z;
-        if (k < n_w) reinterpret_cast<float4*>(v.weight)[b * n_w + k] = z;
-        if (v.storage == kStoreF32) {
-            reinterpret_cast<float4*>(v.r)[b * n_t + k] = z;
-            reinterpret_cast<float4*>(v.g)[b * n_t + k] = z;
-            reinterpret_cast<float4*>(v.b)[b * n_t + k] = z;
-        }
-    }
+// Zero one 512-voxel block's span of an array of ELEM-byte voxels, by the
+// whole CTA in 16-byte stores.
+template <int ELEM>
+__device__ __forceinline__ void zero_block(void* arr, int32_t b) {
+    constexpr int kVec = kBlockVoxels * ELEM / 16;
+    float4* p = reinterpret_cast<float4*>(arr) + (size_t)b * kVec;
+    for (int k = threadIdx.x; k < kVec; k += blockDim.x) p[k] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
-// Zero the first n_voxels voxels of every array of the volume's storage, 16
-// bytes per store (n_voxels is a multiple of 512).
-__global__ void reset_voxels_kernel(DevVolume v, size_t n_voxels) {
-    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-    const size_t n_t = n_voxels * (size_t)tsdf_bytes(v.storage) / 16;
-    const size_t n_w = n_voxels * (size_t)weight_bytes(v.storage) / 16;
-    const bool rgb = v.storage == kStoreF32;
-    for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < n_t;
-         k += (size_t)gridDim.x * blockDim.x) {
-        reinterpret_cast<float4*>(v.tsdf)[k] = z;
-        if (k < n_w) reinterpret_cast<float4*>(v.weight)[k] = z;
-        if (rgb) {
-            reinterpret_cast<float4*>(v.r)[k] = z;
-            reinterpret_cast<float4*>(v.g)[k] = z;
-            reinterpret_cast<float4*>(v.b)[k] = z;
+// Reset: the allocated blocks' voxels to zero (pool indices 0..*count-1, or
+// the *count entries of a list), then the table's slots to empty. The count
+// is read on the device, so the host need not wait for it first. Bound by
+// the stores: 16 bytes per slot and 20 (FP32) per voxel of the blocks.
+template <int S>
+__global__ void __launch_bounds__(kResetThreads) reset_kernel(DevVolume v, const int32_t* list, const int32_t* count) {
+    const int32_t n = min(*count, v.pool_capacity);
+    for (int32_t i = blockIdx.x; i < n; i += gridDim.x) {
+        const int32_t b = list ? list[i] : i;
+        zero_block<tsdf_bytes(S)>(v.tsdf, b);
+        zero_block<weight_bytes(S)>(v.weight, b);
+        if constexpr (S == kStoreF32) {
+            zero_block<4>(v.r, b);
+            zero_block<4>(v.g, b);
+            zero_block<4>(v.b, b);
         }
     }
+    const uint32_t size = v.hash_mask + 1;
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < size; k += gridDim.x * blockDim.x)
+        reinterpret_cast<int4*>(v.table)[k] = make_int4(-1, -1, -1, 0);  // kEmptyKey, no index
 }
+static_assert(kEmptyKey == -1, "an empty slot's key is all ones");
 
 }  // namespace
 
@@ -523,16 +518,14 @@ cudaError_t launch_list_blocks(const DevVolume& v, int32_t* out, int32_t* count,
     return cudaGetLastError();
 }
 
-cudaError_t launch_reset_voxels(const DevVolume& v, int32_t n_blocks, const int32_t* list, cudaStream_t s) {
-    if (n_blocks <= 0) return cudaSuccess;
-    if (list) {
-        reset_listed_kernel<<<n_blocks, 128, 0, s>>>(v, list, n_blocks);
-        return cudaGetLastError();
+cudaError_t launch_reset(const DevVolume& v, const int32_t* list, const int32_t* count, cudaStream_t s) {
+    // One wave of 16 CTAs per SM, striding over the blocks and the slots.
+    const int grid = 148 * 16;
+    switch (v.storage) {
+        case kStoreF16U16: reset_kernel<kStoreF16U16><<<grid, kResetThreads, 0, s>>>(v, list, count); break;
+        case kStoreF64: reset_kernel<kStoreF64><<<grid, kResetThreads, 0, s>>>(v, list, count); break;
+        default: reset_kernel<kStoreF32><<<grid, kResetThreads, 0, s>>>(v, list, count);
     }
-    const size_t n_voxels = (size_t)n_blocks * kBlockVoxels;
-    const size_t n_vec = n_voxels * (size_t)tsdf_bytes(v.storage) / 16;
-    const int grid = (int)std::min<size_t>((n_vec + 255) / 256, (size_t)148 * 16);
-    reset_voxels_kernel<<<grid, 256, 0, s>>>(v, n_voxels);
     return cudaGetLastError();
 }
 

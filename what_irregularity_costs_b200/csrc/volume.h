@@ -106,6 +106,13 @@ struct UpdateScratch {
     uint32_t tag = 0;               // this update's number (never 0)
 };
 
+// A volume's counters, one allocation (a reset clears them together).
+struct VolumeCounters {
+    unsigned long long drop_count;
+    int32_t block_count;
+    uint32_t status;
+};
+
 class Volume {
 public:
     // layout: kLayoutPool (the reference's: pool indices from a counter) or
@@ -195,6 +202,8 @@ public:
     // step on stream s (takes the next update number).
     bool reserve_batch(int32_t max_points);
     SceneWork batch_work(const BatchArgs& a, cudaStream_t s);
+    // A batched step did not queue all of its passes.
+    void mark_unfinished() { unfinished_ = true; }
 
     // Timing.
     void set_timing(bool on) { timing_ = on; }
@@ -218,6 +227,10 @@ private:
     bool ok_ = false;
     int device_ = -1;
     DevVolume dv_{};
+    VolumeCounters* counters_ = nullptr;  // device
+    // An update that did not queue all of its passes may have left per-voxel
+    // batch state behind: the next reset clears all of it.
+    bool unfinished_ = false;
     float weight_cap_ = 0.0f;
     cudaStream_t stream_ = nullptr;
     UpdateScratch us_{};
@@ -289,8 +302,9 @@ cudaError_t launch_rebuild_table(const DevVolume& v, int32_t n_blocks, cudaStrea
 // The voxel arrays of a storage mode (tsdf, weight[, r, g, b]) and their
 // bytes per voxel; returns how many (snapshot.cu).
 size_t voxel_arrays(int storage, const DevVolume& d, void* out[5], size_t bytes[5]);
-// Zero the voxels of n blocks: pool indices 0..n-1, or those of a list.
-cudaError_t launch_reset_voxels(const DevVolume& v, int32_t n_blocks, const int32_t* list, cudaStream_t s);
+// Empty the table and zero the voxels of the allocated blocks: pool indices
+// 0..*count-1, or the *count entries of a list (count: device memory).
+cudaError_t launch_reset(const DevVolume& v, const int32_t* list, const int32_t* count, cudaStream_t s);
 // List the occupied slots of the table (slot-index layout) into out.
 cudaError_t launch_list_blocks(const DevVolume& v, int32_t* out, int32_t* count, cudaStream_t s);
 // Extraction over n blocks: pool indices 0..n-1, or those of a list.
