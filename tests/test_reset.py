@@ -39,10 +39,20 @@ def test_reset_volume_is_a_new_one(cuda, storage, layout, size):
     for v in (vol, new):
         for p, f in zip(points, frames):
             v.integrate(p, f.cam)
+    # Read out by coordinate, in the arrays' own types (whole volumes, so that
+    # both layouts read alike; slots in use have a key).
     out = []
     for v in (vol, new):
-        coords, mean, weight = v.means()
-        order = np.lexsort(coords.T[::-1])
-        out.append((coords[order], mean[order], weight[order]))
+        v.synchronize()
+        view = v.device_view()
+        n = view.pool_capacity
+        coords = device_tensor(view.block_coord, (n, 3), "<i4").cpu().numpy()
+        if layout == LAYOUT_SLOT_INDEX:
+            used = np.nonzero(v.table()[0] >= 0)[0]
+        else:
+            used = np.arange(v.block_count())
+        used = used[np.lexsort(coords[used].T[::-1])]
+        out.append([coords[used]] + [device_tensor(ptr, (n, 512), typ).cpu().numpy()[used]
+                                     for ptr, typ in zip((view.tsdf, view.weight), TYPES[storage])])
     for a, b in zip(*out):
         assert np.array_equal(a, b)

@@ -8,25 +8,26 @@
 //
 // One thread walks one point's band (2*steps+1 samples, kChunk at a time in
 // registers); a persistent grid of CTAs strides over tiles of 128
-// consecutive points (neighbouring pixels of a frame). Along a ray the block
-// changes rarely, so a thread keeps the runs of equal blocks of its chunk
-// (their keys in a per-thread column of shared memory) and resolves each
-// once. The resolution is warp-cooperative: for each run index the warp's
-// lanes group equal block keys with __match_any_sync and only the lowest lane
-// of a group probes the global table (and inserts), leaving the pool index in
-// shared memory for the group -- neighbouring pixels share blocks, so the
-// table sees a fraction of the per-sample probes and far fewer contending CAS
-// attempts on a new block. The groups of all run indices are formed first and
-// each leader then resolves its runs with their home-slot probes in flight
-// together, so a chunk waits for about one table access, not one per run.
+// consecutive points (neighbouring pixels of a frame). The blocks of a warp's
+// samples are resolved through a small table in shared memory (band_point):
+// every distinct block of the 32 points is probed once, by one lane, with all
+// of the warp's probes (the first two slots of each key's sequence) in flight
+// together, so the global table sees a fraction of the per-sample probes and
+// far fewer contending CAS attempts on a new block.
 //
-// Update tail. The group leader also tags the block as touched by this update
-// (one atomic exchange unless a cached read already shows the tag; the first
-// tagger appends it to the touched list).
+// What bounds it (four 640x480 frames a call): L1 throughput of the scattered
+// weight gathers and reductions (about 21 M sectors, one a cycle per SM: 75
+// us) and instruction issue (53.6 M warp instructions: 48 us); 122 us
+// measured, 143 before the table (67.1 M instructions, and values spilled
+// around calls).
+//
+// Update tail. The resolving lane also tags the block as touched by this update
+// (one atomic exchange on the spare word of its table slot, unless the probe
+// already showed the tag; the first tagger appends it to the touched list).
 // Every band sample whose voxel can still accept a contribution adds one to
 // the voxel's batch count and its normalised SDF, in 2^-40 fixed point, to
 // the voxel's 64-bit sum: fire-and-forget L2 reductions, whose order does not
-// matter, issued once per run of consecutive lanes that share the voxel. Every band slot (point i, step s) also gets a 4-byte record at
+// matter. Every band slot (point i, step s) also gets a 4-byte record at
 // records[(s + steps) * n + i] -- step-major, so each store of a warp is one
 // contiguous 128-byte line -- holding the voxel's global index or kNoVoxel;
 // only voxels that cross the cap read them again (their canonical order is
@@ -56,18 +57,13 @@ static_assert(kBandThreads >= kMaxBatchScenes, "one thread per scene builds the 
 #define OSN_BAND_CHUNK 9
 #endif
 constexpr int kChunk = OSN_BAND_CHUNK;  // samples per ray held in registers (9: the whole band at 4 voxels)
-// Resident CTAs per SM the register budget is sized for. The several-frame
-// and batched walks: 7 (72 registers), measured 1.4 % faster on the room
-// trajectory than 8 (64 registers) and 6; the one-frame walk: 8 (at 7 it
-// measured 6 % slower, its batches are a third of the size).
+// Resident CTAs per SM the register budget is sized for: 6 (80 registers,
+// nothing spilled). Four 640x480 frames per call took 121 us at 6, 124 at 7
+// (72 registers), 131 at 8 (64); one frame 43.8 us at 6, 44.9 at 8.
 #ifndef OSN_BAND_MIN_BLOCKS
-#define OSN_BAND_MIN_BLOCKS 8
-#endif
-#ifndef OSN_BAND_FRAMES_MIN_BLOCKS
-#define OSN_BAND_FRAMES_MIN_BLOCKS 7
+#define OSN_BAND_MIN_BLOCKS 6
 #endif
 constexpr int kBandMinBlocks = OSN_BAND_MIN_BLOCKS;
-constexpr int kBandFramesMinBlocks = OSN_BAND_FRAMES_MIN_BLOCKS;
 
 // Band records and slot values are read once more, by the group pass of the
 // same update: stored with the streaming hint (1, evict-first) or as
@@ -90,22 +86,28 @@ __device__ __forceinline__ void store_slot(T* p, T x) {
     else *p = x;
 }
 
-// Per-sample state: voxel within block (9 bits), run index (4 bits), valid.
-constexpr uint32_t kLvMask = 0x1FFu;
-constexpr int kRunShift = 9;
-constexpr uint32_t kValid = 1u << 30;
+// A block's pool index (-1: absent or dropped) and the slot that holds its key.
+struct Resolved {
+    int32_t bi;
+    uint32_t slot;
+};
 
 template <int MODE>
-__device__ __forceinline__ int32_t resolve(const DevVolume& v, long long key,
-                                           unsigned long long* hist, int n_bins) {
+__device__ __forceinline__ Resolved resolve(const DevVolume& v, long long key,
+                                            unsigned long long* hist, int n_bins) {
     const int bx = unpack_axis(key, 2 * kCoordBits);
     const int by = unpack_axis(key, kCoordBits);
     const int bz = unpack_axis(key, 0);
-    if (MODE == kLookupOnly) return find_block(v, bx, by, bz, key);
+    const uint32_t home = hash_slot(bx, by, bz, v.hash_mask);
+    if (MODE == kLookupOnly) {
+        uint32_t probes = 0;
+        const int32_t bi = find_block(v, bx, by, bz, key, probes);
+        return Resolved{bi, (home + probes - 1u) & v.hash_mask};
+    }
     const InsertResult r = find_or_insert<MODE>(v, bx, by, bz, key);
     if (MODE == kAllocProbeHist && n_bins > 0)
         atomicAdd(&hist[min(r.probes, (uint32_t)(n_bins - 1))], 1ull);
-    return r.idx;
+    return Resolved{r.idx, (home + r.probes - 1u) & v.hash_mask};
 }
 
 // Modes whose first probe may be answered from the block's home slot alone.
@@ -114,77 +116,92 @@ __device__ __forceinline__ constexpr bool has_fast_probe() {
     return MODE == kAllocInsert || MODE == kLookupOnly;
 }
 
-// The block's home-slot entry, through L1. A slot goes empty -> claimed
-// (key, -1) -> published (key, index) and never changes again within an
-// update, so an entry that shows this key with a valid index is final, and
-// with no concurrent insertion (lookup) an empty home slot means absent.
-template <int MODE>
-__device__ __forceinline__ int4 home_entry(const DevVolume& v, long long key) {
-    if (!has_fast_probe<MODE>()) return make_int4(0, 0, -1, 0);
-    const uint32_t h = hash_slot(unpack_axis(key, 2 * kCoordBits), unpack_axis(key, kCoordBits),
-                                 unpack_axis(key, 0), v.hash_mask);
-    const int4* e = reinterpret_cast<const int4*>(&v.table[h]);
-    return MODE == kLookupOnly ? __ldg(e) : __ldca(e);
+constexpr int32_t kUnsettled = -2;  // the full probe is needed
+
+// The home slot of a packed key, from the key's words (x: low, y: high).
+__device__ __forceinline__ uint32_t home_slot(const DevVolume& v, uint2 key) {
+    constexpr uint32_t kMask = (1u << kCoordBits) - 1u, kBias = (uint32_t)kCoordBias;
+    const uint32_t bz = (key.x & kMask) - kBias;
+    const uint32_t by = (__funnelshift_r(key.x, key.y, kCoordBits) & kMask) - kBias;
+    const uint32_t bx = (key.y >> (2 * kCoordBits - 32)) - kBias;
+    return (bx * 73856093u ^ by * 19349663u ^ bz * 83492791u) & v.hash_mask;
 }
 
-// The pool index the home entry settles, or -2 when the full probe is needed.
+// The first two slots of a key's probe sequence, both loads in flight
+// together, and what they settle: the pool index (and slot) of the key, -1
+// when it is absent (lookups), else kUnsettled. A slot goes empty -> claimed
+// (key, -1) -> published (key, index) and its key and index never change again
+// within an update, so an entry read through L1 that shows this key with a
+// valid index is final, wherever it is; and with no concurrent insertion
+// (lookup) an empty slot ends the sequence. The hash sends 16 % of a room's
+// blocks to their second slot: nearly every warp meets one of them.
+struct Probe {
+    int4 e0, e1;
+};
 template <int MODE>
-__device__ __forceinline__ int32_t settle_home(const DevVolume& v, int4 raw, long long key) {
-    if (!has_fast_probe<MODE>()) return -2;
-    const long long k0 = ((long long)(unsigned)raw.y << 32) | (unsigned)raw.x;
-    if (k0 == key && raw.z >= 0 && raw.z < v.pool_capacity) return raw.z;
-    if (MODE == kLookupOnly && k0 == kEmptyKey) return -1;
-    return -2;
+__device__ __forceinline__ Probe probe_start(const DevVolume& v, uint32_t home) {
+    Probe p{make_int4(0, 0, -1, 0), make_int4(0, 0, -1, 0)};
+    if (has_fast_probe<MODE>()) {
+        p.e0 = __ldca(reinterpret_cast<const int4*>(&v.table[home]));
+        p.e1 = __ldca(reinterpret_cast<const int4*>(&v.table[(home + 1u) & v.hash_mask]));
+    }
+    return p;
+}
+// Sets out (slot: the home slot on entry); returns the touch tag seen.
+template <int MODE>
+__device__ __forceinline__ uint32_t probe_settle(const DevVolume& v, const Probe& p, uint2 key, Resolved& out) {
+    out.bi = kUnsettled;
+    if (!has_fast_probe<MODE>()) return 0u;
+    const bool at0 = (uint32_t)p.e0.x == key.x && (uint32_t)p.e0.y == key.y;
+    const bool at1 = !at0 && (uint32_t)p.e1.x == key.x && (uint32_t)p.e1.y == key.y;
+    const int32_t idx = at1 ? p.e1.z : p.e0.z;
+    if ((at0 || at1) && (uint32_t)idx < (uint32_t)v.pool_capacity) {
+        out.bi = idx;
+        if (at1) out.slot = (out.slot + 1u) & v.hash_mask;
+    } else if (MODE == kLookupOnly && ((p.e0.x & p.e0.y) == -1 || (!at0 && (p.e1.x & p.e1.y) == -1))) {
+        out.bi = -1;  // kEmptyKey before the key
+    }
+    return (uint32_t)(at1 ? p.e1.w : p.e0.w);
 }
 
-// The full probe (and insertion) protocol, out of line: it is the rare path
-// of the fast-probe modes and keeps their walk loop in registers.
+// The full probe for the lanes with `need` set (called by the whole warp):
+// equal keys are grouped across the warp and one leader per key probes.
 template <int MODE>
-__device__ __noinline__ int32_t resolve_slow(HashEntry* table, uint32_t hash_mask, int32_t pool,
-                                             int32_t* block_count, unsigned long long* drop_count,
-                                             BlockCoord* block_coord, uint32_t* status,
-                                             int32_t spin_limit, int32_t* block_chunk, int32_t chunk,
-                                             int32_t slot_index, long long key) {
-    DevVolume v{};
-    v.table = table;
-    v.hash_mask = hash_mask;
-    v.pool_capacity = pool;
-    v.block_count = block_count;
-    v.drop_count = drop_count;
-    v.block_coord = block_coord;
-    v.status = status;
-    v.spin_limit = spin_limit;
-    v.block_chunk = block_chunk;
-    v.chunk = chunk;
-    v.slot_index = slot_index;
-    return resolve<MODE>(v, key, nullptr, 0);
-}
-
-template <int MODE>
-__device__ __forceinline__ int32_t resolve_from(const DevVolume& v, int4 raw, long long key,
+__device__ __forceinline__ void resolve_grouped(const DevVolume& v, bool need, long long key, Resolved& out,
                                                 unsigned long long* hist, int n_bins) {
-    if (!has_fast_probe<MODE>()) return resolve<MODE>(v, key, hist, n_bins);
-    const int32_t bi = settle_home<MODE>(v, raw, key);
-    if (bi != -2) return bi;
-    return resolve_slow<MODE>(v.table, v.hash_mask, v.pool_capacity, v.block_count, v.drop_count,
-                              v.block_coord, v.status, v.spin_limit, v.block_chunk, v.chunk, v.slot_index,
-                              key);
+    const unsigned want = __ballot_sync(0xffffffffu, need);
+    if (want == 0u) return;
+    if (need) {
+        const int leader = __ffs(__match_any_sync(want, key)) - 1;
+        Resolved r{-1, 0u};
+        if (leader == (int)(threadIdx.x & 31)) r = resolve<MODE>(v, key, hist, n_bins);
+        out.bi = __shfl_sync(want, r.bi, leader);
+        out.slot = __shfl_sync(want, r.slot, leader);
+    }
+    __syncwarp();
 }
 
-// Tag a block as touched by this update; the first tagger appends it to the
-// touched list. A cached read that already shows the tag saves the exchange
-// (a stale read can only show an older tag). The appends of the lanes that
-// arrive together take their places with one atomic on the list's counter.
-__device__ __forceinline__ void tag_touched(const UpdateScratch& u, int32_t bi, uint32_t seen) {
-    const bool add = bi >= 0 && seen != u.tag && atomicExch(&u.blk_touch[bi], u.tag) != u.tag;
-    const unsigned act = __activemask();
-    const unsigned want = __ballot_sync(act, add);
-    if (!want) return;
-    const int ldr = __ffs(want) - 1;
+// Tag the blocks of the lanes with `need` set as touched by this update (the
+// tag is the spare word of the block's table slot); the first tagger of a
+// block appends it to the touched list. Called by the whole warp where any
+// lane saw an older tag: one lane per block exchanges (SHARED: lanes may hold
+// the same block), and the appends of the warp take their places with one
+// atomic on the list's counter.
+template <bool SHARED>
+__device__ __forceinline__ void tag_touched(const DevVolume& v, const UpdateScratch& u, bool need, int32_t bi,
+                                            uint32_t slot) {
+    const unsigned want = __ballot_sync(0xffffffffu, need);
+    if (want == 0u) return;
+    const int lane = (int)(threadIdx.x & 31);
+    bool add = false;
+    if (need && (!SHARED || __ffs(__match_any_sync(want, bi)) - 1 == lane))
+        add = (uint32_t)atomicExch(&v.table[slot].pad, (int)u.tag) != u.tag;
+    const unsigned adds = __ballot_sync(0xffffffffu, add);
+    if (adds == 0u) return;
     int base = 0;
-    if ((int)(threadIdx.x & 31) == ldr) base = atomicAdd(&u.ctl->n_touched, __popc(want));
-    base = __shfl_sync(act, base, ldr);
-    if (add) u.touched[base + __popc(want & lanemask_lt())] = bi;
+    if (lane == __ffs(adds) - 1) base = atomicAdd(&u.ctl->n_touched, __popc(adds));
+    base = __shfl_sync(0xffffffffu, base, __ffs(adds) - 1);
+    if (add) u.touched[base + __popc(adds & lanemask_lt())] = bi;
 }
 
 // Fire-and-forget L2 reductions (no value comes back, nothing waits).
@@ -195,168 +212,376 @@ __device__ __forceinline__ void red_add(unsigned long long* p, unsigned long lon
     asm volatile("red.global.add.u64 [%0], %1;" ::"l"(p), "l"(x));
 }
 
-// Shared memory of one band CTA: per-thread run columns, run q of thread t
-// at [q][t] (no bank conflicts).
+// Shared memory of one band CTA.
+//   table    per warp: the blocks of its samples (x: key within the warp, y:
+//            pool index)
+//   run_key  measurement modes: per-thread columns of run keys (x: low word),
+//            run q of thread t at [q][t] (no bank conflicts)
+constexpr int kTableEntries = 64;  // two per lane
+template <bool MEASURE>
 struct BandSmem {
-    long long run_key[kChunk][kBandThreads];
-    int32_t run_bi[kChunk][kBandThreads];   // written by the run's group leader
-    uint8_t run_src[kChunk][kBandThreads];  // leader lane of the run's group
+    uint2 table[MEASURE ? 1 : kBandThreads / 32][kTableEntries];
+    uint2 run_key[MEASURE ? kChunk : 1][kBandThreads];
 };
 
-// Walk point i (already loaded into px, py, pz; i >= a.n for lanes without a
-// point) through its band: runs, warp-cooperative block resolution, then
-// the update tail. Called by every thread of the CTA, warp-synchronously.
-// Block resolution schemes of the band walk.
-constexpr int kProbeWarp = 0;  // equal keys grouped across the warp, one leader probes
-constexpr int kProbeLane = 1;  // every lane probes its own runs (L1 shares the loads)
+// N consecutive band samples of a ray once their blocks are resolved: the
+// voxels' weights gathered together, then the saturation gate, counts, sums
+// and records. vox: the samples' voxels or kNoVoxel; dsq: squared distance of
+// camera and voxel centre (unfused float arithmetic, as the reference's), from
+// which the signed distance is taken only where a lane counts; f64: the FP64
+// oracle's value of sample j. n_steps: samples in use (warp-uniform). writes:
+// this lane's records are stored.
+template <int S, int N, typename F64>
+__device__ __forceinline__ void count_samples(const DevVolume& v, const UpdateScratch& u, bool writes,
+                                              uint32_t stride, float dist, uint32_t (&vox)[N],
+                                              const float (&dsq)[N], int n_steps, uint32_t& slot,
+                                              uint32_t& counted, const F64& f64) {
+    // Without a cap no voxel can be full or cross it: no weight is looked at,
+    // and no record is kept for the cap selection.
+    const bool capped = v.weight_cap > 0.0f;
+    if (capped) {
+        float w0[N];
+#pragma unroll
+        for (int j = 0; j < N; ++j) w0[j] = weight_at<S>(v, vox[j] == kNoVoxel ? 0u : vox[j]);
+#pragma unroll
+        for (int j = 0; j < N; ++j)
+            if (w0[j] >= v.weight_cap) vox[j] = kNoVoxel;  // takes no contribution
+    }
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        if (j >= n_steps) break;
+        const bool counts = vox[j] != kNoVoxel;
+        if (__any_sync(0xffffffffu, counts)) {
+            long long fix;
+            float sdf_n = 0.0f;
+            if constexpr (S == kStoreF64) {
+                fix = counts ? f64(j) : 0ll;
+            } else {
+                const float sdf = __fsub_rn(dist, __fsqrt_rn(dsq[j]));
+                sdf_n = fminf(fmaxf(__fmul_rn(sdf, v.inv_trunc), -1.0f), 1.0f);
+                fix = to_fix(sdf_n);
+            }
+            if (counts) {
+                // Kept for the records of voxels that cross the cap, so the
+                // update tail never reads the batch's points again.
+                if (S != kStoreF64 && capped) store_slot(u.slot_val + slot, sdf_n);
+                red_add(&u.vcnt[vox[j]], 1u);
+                red_add(&u.vacc[vox[j]], (unsigned long long)fix);
+                ++counted;
+            }
+        }
+        if (capped && writes) store_slot(u.records + slot, vox[j]);  // read again by the group pass
+        slot += stride;
+    }
+}
 
+// The FP64 oracle's normalised SDF of voxel (vx, vy, vz), 2^-40 fixed point.
+__device__ __forceinline__ long long oracle_fix(const DevVolume& v, const BatchArgs& a, const Ray& r, int vx,
+                                                int vy, int vz) {
+    return to_fix(clamp_sdf_n_f64(sdf_f64(v, a, r.px, r.py, r.pz, vx, vy, vz), v.trunc));
+}
+
+// The allocate-only walk of the measurement modes: every lane keeps the runs
+// of equal blocks of a chunk of its samples (their keys in a column of shared
+// memory), and each run index of the warp's lanes is resolved by the full
+// probe, one leader per distinct key. Returns the samples dropped.
+template <int MODE>
+__device__ __forceinline__ uint32_t measure_point(const DevVolume& v, const Ray& r, bool live, uint2 (*run_key)[kBandThreads],
+                                                  unsigned long long* hist, int n_bins) {
+    const int t = threadIdx.x;
+    uint32_t drops = 0u;
+    for (int c0 = -v.steps; c0 <= v.steps; c0 += kChunk) {
+        int n_run = 0, n_of[kChunk];  // samples of each run
+        int ox = 0, oy = 0, oz = 0;   // the last valid sample's voxel
+#pragma unroll
+        for (int j = 0; j < kChunk; ++j) n_of[j] = 0;
+#pragma unroll
+        for (int j = 0; j < kChunk; ++j) {
+            int vx, vy, vz;
+            float dsq;
+            if (live && c0 + j <= v.steps && band_sample_ray(v, r, c0 + j, vx, vy, vz, dsq)) {
+                // A straight ray leaves a block (a convex box) for good, so
+                // equal consecutive blocks are the only repeats.
+                if (n_run == 0 || (((vx ^ ox) | (vy ^ oy) | (vz ^ oz)) >> 3) != 0) {
+                    const unsigned long long k = (unsigned long long)pack_key(vx >> 3, vy >> 3, vz >> 3);
+                    run_key[n_run][t] = make_uint2((uint32_t)k, (uint32_t)(k >> 32));
+                    ++n_run;
+                }
+                ox = vx;
+                oy = vy;
+                oz = vz;
+#pragma unroll
+                for (int q = 0; q < kChunk; ++q) n_of[q] += q == n_run - 1 ? 1 : 0;
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < kChunk; ++q) {
+            if (!__any_sync(0xffffffffu, q < n_run)) break;
+            const uint2 k2 = q < n_run ? run_key[q][t] : make_uint2(0u, 0u);
+            Resolved res{0, 0u};
+            resolve_grouped<MODE>(v, q < n_run, (long long)((unsigned long long)k2.y << 32 | k2.x), res, hist, n_bins);
+            if (res.bi < 0) drops += (uint32_t)n_of[q];
+        }
+        __syncwarp();  // the run columns are rewritten by the next chunk
+    }
+    return drops;
+}
+
+// Limits of the fast walk, in voxels. Coordinates below kReach: the floor is
+// exact and block coordinates fit a key. Below kSureReach, rounding errors
+// are small against a voxel, which the occlusion shortcut assumes. Samples
+// within kSpreadXY / kSpreadZ of the warp's first point: their offsets fit.
+constexpr float kReach = 2097152.0f;
+constexpr float kSureReach = 32768.0f;
+constexpr float kSpreadXY = 1000.0f;
+constexpr float kSpreadZ = 490.0f;
+constexpr float kFloorMagic = 12582912.0f;  // 1.5 * 2^23
+constexpr uint32_t kFloorBits = 0x4B400000u;  // its bits
+constexpr uint32_t kNoOffset = 0xFFFFFFFFu;  // no sample; no block
+
+// A voxel's offset from the warp's origin (block-aligned; 1024, 1024 and 512
+// voxels before the first point's block): x (11 bits), y << 11 (11 bits),
+// z << 22 (10 bits). An offset without the low three bits of its fields is
+// its block's key within the warp.
+__device__ __forceinline__ uint32_t pack_offset(uint32_t x, uint32_t y, uint32_t z) {
+    return x + (y << 11) + (z << 22);
+}
+constexpr uint32_t kOffsetBlock = ~(7u | 7u << 11 | 7u << 22);
+// The block's entry in the warp's table: its coordinates modulo 4, so the
+// blocks of any 4 x 4 x 4 neighbourhood have entries of their own. One
+// product brings the fields together (no two of its partial products meet).
+__device__ __forceinline__ uint32_t table_entry(uint32_t w) {
+    return ((w & (3u << 3 | 3u << 14 | 3u << 25)) * (1u << 23 | 1u << 14 | 1u << 5)) >> 26;
+}
+// The offset's voxel within its block, (lz * 8 + ly) * 8 + lx, in the nine
+// high bits; the same way.
+__device__ __forceinline__ uint32_t voxel_high(uint32_t w) {
+    return (w & (7u | 7u << 11 | 7u << 22)) * (1u << 23 | 1u << 15 | 1u << 7);
+}
+
+// Walk point i (already loaded into px, py, pz; i >= a.n for lanes without a
+// point) through its band. Called by every thread of the CTA,
+// warp-synchronously.
+//
+// The 32 points of a warp are neighbouring pixels, so a chunk of their bands
+// lies in a few blocks (12 in the median 640x480 frame). Each sample writes
+// its block's key into the warp's table in shared memory; lane l then
+// resolves the blocks found in entries l and l + 32, all in one round trip:
+// every distinct block of the warp is probed once, and no key is matched
+// across lanes. A sample that finds another block's key in its entry goes
+// another round. Nothing is called out of line: values that live across a
+// call were spilled at every use (148 local loads a tile, a third of the
+// walk's time).
+//
+// Samples round exactly as band_sample's: floor(x) is taken by adding
+// 1.5 * 2^23 with rounding toward -infinity (exact for |x| < 2^22; the low
+// bits are then the voxel coordinate), and (vf + 0.5) * size is the single
+// fused rounding of vf * size + size / 2 (vf + 0.5 is exact). Within
+// kSureReach, a sample up to step trunc / voxel - 1 (v.sure_step) cannot be
+// occluded: its voxel's centre lies within 0.87 voxels of it and rounding
+// errors stay below 0.1 voxels.
+//
 // FRAMES: the batch holds several frames; (cx, cy, cz) is the camera of
 // point i's frame (otherwise the batch's one camera is used).
-template <int MODE, bool RECORDS, int S, int PROBE = kProbeWarp, bool FRAMES = false>
+template <int MODE, bool RECORDS, int S, bool FRAMES = false>
 __device__ __forceinline__ void band_point(const DevVolume& v, const BatchArgs& a, const UpdateScratch& u,
-                                           int i, bool has, float px, float py, float pz, BandSmem& sm,
-                                           uint32_t& drops, uint32_t& counted,
+                                           int i, bool has, float px, float py, float pz,
+                                           BandSmem<!has_fast_probe<MODE>()>& sm, uint32_t& drops, uint32_t& counted,
                                            unsigned long long* hist, int n_bins, float cx = 0.0f,
                                            float cy = 0.0f, float cz = 0.0f) {
     static_assert(!(FRAMES && S == kStoreF64), "the FP64 oracle integrates one frame per batch");
-    const int t = threadIdx.x;
-    const int lane = t & 31, wbase = t & ~31;
     const bool counts_drops = MODE != kLookupOnly && MODE != kAllocNoCas && MODE != kAllocCountingCas;
-    const bool sat_check = RECORDS && v.weight_cap > 0.0f;
-    auto& run_key = sm.run_key;
-    auto& run_bi = sm.run_bi;
-    auto& run_src = sm.run_src;
+    if (!FRAMES) {
+        cx = a.cam_x;
+        cy = a.cam_y;
+        cz = a.cam_z;
+    }
     Ray r;
-    const bool live = i < a.n && has &&
-                      (FRAMES ? ray_setup_cam(a.radius_sq, cx, cy, cz, px, py, pz, r)
-                              : ray_setup_at(a, px, py, pz, r));
-    uint32_t* rec = RECORDS ? u.records + i : nullptr;  // slot (s = -steps, i)
+    const bool in_batch = i < a.n;
+    const bool live = in_batch && has && ray_setup_cam(a.radius_sq, cx, cy, cz, px, py, pz, r);
 
-    for (int c0 = -v.steps; c0 <= v.steps; c0 += kChunk) {
-        uint32_t st[kChunk];
-        float sd[kChunk];
-        int n_run = 0;
-        long long last = kNoKey;
+    if constexpr (!has_fast_probe<MODE>()) {
+        const uint32_t d = measure_point<MODE>(v, r, live, sm.run_key, hist, n_bins);
+        if (counts_drops) drops += d;
+        return;
+    }
 
-        // Phase 1: the chunk's samples; runs of equal blocks in walk order.
-#pragma unroll
-        for (int j = 0; j < kChunk; ++j) {
-            st[j] = 0u;
-            sd[j] = 0.0f;
-            const int s = c0 + j;
-            int vx, vy, vz;
-            float sdf;
-            if (live && s <= v.steps &&
-                (FRAMES ? band_sample_ray(v, r, s, vx, vy, vz, sdf) : band_sample(v, a, r, s, vx, vy, vz, sdf))) {
-                const int bx = vx >> 3, by = vy >> 3, bz = vz >> 3;  // floor_div(v, 8)
-                const long long key = pack_key(bx, by, bz);
-                // A straight ray leaves a block (a convex box) for good, so
-                // equal consecutive keys are the only repeats.
-                if (key != last) {
-                    last = key;
-                    run_key[n_run][t] = key;
-                    ++n_run;
-                }
-                const uint32_t lv =
-                    (uint32_t)(((vz & 7) * kBlockDim + (vy & 7)) * kBlockDim + (vx & 7));
-                st[j] = kValid | lv | (uint32_t)(n_run - 1) << kRunShift;
-                sd[j] = sdf;
-            }
-        }
+    const int lane = threadIdx.x & 31;
+    uint2* const table = sm.table[threadIdx.x >> 5];
+    const float half = __fmul_rn(0.5f, v.voxel_size);
+    const float far = v.inv_voxel * (fmaxf(fmaxf(fabsf(px), fabsf(py)), fabsf(pz)) +
+                                     fmaxf(fmaxf(fabsf(cx), fabsf(cy)), fabsf(cz)));
+    const float band = (float)v.steps + 2.0f;
+    unsigned todo = __ballot_sync(0xffffffffu, live);
+    // Usually one round: every live lane's samples fit the offsets from the
+    // first lane's block. Lanes too far away from it go another round.
+    int round = 0;
+    for (; round == 0 || todo != 0u; ++round) {
+        const int first = todo ? __ffs(todo) - 1 : 0;
+        const float fx = __shfl_sync(0xffffffffu, px, first), fy = __shfl_sync(0xffffffffu, py, first),
+                    fz = __shfl_sync(0xffffffffu, pz, first);
+        const bool mine = ((todo >> lane) & 1u) && far < kReach &&
+                          v.inv_voxel * fmaxf(fabsf(px - fx), fabsf(py - fy)) + band < kSpreadXY &&
+                          v.inv_voxel * fabsf(pz - fz) + band < kSpreadZ;
+        const unsigned group = __ballot_sync(0xffffffffu, mine);
+        if (todo != 0u && (group == 0u || round == 3)) break;  // warp-uniform
+        // Steps up to this one need no occlusion test.
+        const int sure_step = __all_sync(0xffffffffu, far < kSureReach || !mine) ? v.sure_step : INT_MIN;
+        const bool writes = mine || (round == 0 && in_batch && !live);
+        uint32_t slot = (uint32_t)i;  // band slot (s = -steps, i)
+        // The warp's origin as raw floor bits.
+        const uint32_t ox = (__float_as_uint(__fadd_rd(__fmul_rn(fx, v.inv_voxel), kFloorMagic)) & ~7u) - 1024u;
+        const uint32_t oy = (__float_as_uint(__fadd_rd(__fmul_rn(fy, v.inv_voxel), kFloorMagic)) & ~7u) - 1024u;
+        const uint32_t oz = (__float_as_uint(__fadd_rd(__fmul_rn(fz, v.inv_voxel), kFloorMagic)) & ~7u) - 512u;
+        const uint32_t base = pack_offset(ox, oy, oz);
 
-        // Phase 2a: group equal keys across the warp, one round per run
-        // index; the lowest lane of a group leads it. (Per-lane probing: every
-        // lane leads its own runs.)
-        uint32_t lead = 0u;
-        if constexpr (PROBE == kProbeWarp) {
-            for (int q = 0; q < kChunk; ++q) {
-                if (!__any_sync(0xffffffffu, q < n_run)) break;
-                const long long key = q < n_run ? run_key[q][t] : kNoKey;
-                const unsigned grp = __match_any_sync(0xffffffffu, key);
-                const int leader = __ffs(grp) - 1;
-                if (q < n_run) run_src[q][t] = (uint8_t)leader;
-                if (key != kNoKey && lane == leader) lead |= 1u << q;
-            }
-        } else {
-            for (int q = 0; q < n_run; ++q) run_src[q][t] = (uint8_t)lane;
-            lead = n_run ? (1u << n_run) - 1u : 0u;
-        }
-        // Phase 2b: each leader resolves its runs two at a time, both
-        // home-slot probes (and then both tag reads) in flight together.
-        while (lead) {
-            const int qa = __ffs(lead) - 1;
-            lead &= lead - 1u;
-            const int qb = lead ? __ffs(lead) - 1 : -1;
-            if (qb >= 0) lead &= lead - 1u;
-            const long long ka = run_key[qa][t];
-            const long long kb = qb >= 0 ? run_key[qb][t] : kNoKey;
-            const int4 ra = home_entry<MODE>(v, ka);
-            const int4 rb = qb >= 0 ? home_entry<MODE>(v, kb) : make_int4(0, 0, -1, 0);
-            const int32_t ba = resolve_from<MODE>(v, ra, ka, hist, n_bins);
-            const int32_t bb = qb >= 0 ? resolve_from<MODE>(v, rb, kb, hist, n_bins) : -1;
-            run_bi[qa][t] = ba;
-            if (qb >= 0) run_bi[qb][t] = bb;
-            if (RECORDS) {
-                const uint32_t sa = ba >= 0 ? __ldca(&u.blk_touch[ba]) : u.tag;
-                const uint32_t sb = bb >= 0 ? __ldca(&u.blk_touch[bb]) : u.tag;
-                tag_touched(u, ba, sa);
-                tag_touched(u, bb, sb);
-            }
-        }
-        __syncwarp();
-
-        // Phase 3: drops; then every sample's weight gather in flight
-        // together; then the saturation gate, counts, sums and records.
-        uint32_t vox[kChunk];
-#pragma unroll
-        for (int j = 0; j < kChunk; ++j) {
-            vox[j] = kNoVoxel;
-            if (st[j] & kValid) {
-                const uint32_t q = (st[j] >> kRunShift) & 15u;
-                const int32_t bi = run_bi[q][wbase + run_src[q][t]];
-                if (bi < 0) {
-                    if (counts_drops) ++drops;
-                } else {
-                    vox[j] = (uint32_t)bi * kBlockVoxels + (st[j] & kLvMask);
-                }
-            }
-        }
-        if (RECORDS) {
-            float w0[kChunk];
-#pragma unroll
-            for (int j = 0; j < kChunk; ++j)
-                w0[j] = (sat_check && vox[j] != kNoVoxel) ? weight_at<S>(v, vox[j]) : 0.0f;
+        for (int c0 = -v.steps; c0 <= v.steps; c0 += kChunk) {
+            const int n_steps = min(kChunk, v.steps - c0 + 1);  // samples of this chunk
+            table[lane].x = kNoOffset;
+            table[lane + 32].x = kNoOffset;
+            __syncwarp();
+            uint32_t vox[kChunk];  // voxel offset, then the voxel's index
+            float dsq[kChunk];
 #pragma unroll
             for (int j = 0; j < kChunk; ++j) {
-                if (c0 + j > v.steps) break;
-                uint32_t out = kNoVoxel;
-                if (vox[j] != kNoVoxel && !(sat_check && w0[j] >= v.weight_cap)) {
-                    out = vox[j];
-                    long long fix;
-                    if constexpr (S == kStoreF64) {
-                        // The oracle's value of the same sample, in double.
-                        const long long key = run_key[(st[j] >> kRunShift) & 15u][t];
-                        const uint32_t lv = st[j] & kLvMask;
-                        const int vx = unpack_axis(key, 2 * kCoordBits) * kBlockDim + (int)(lv & 7u);
-                        const int vy = unpack_axis(key, kCoordBits) * kBlockDim + (int)((lv >> 3) & 7u);
-                        const int vz = unpack_axis(key, 0) * kBlockDim + (int)(lv >> 6);
-                        fix = to_fix(clamp_sdf_n_f64(sdf_f64(v, a, r.px, r.py, r.pz, vx, vy, vz), v.trunc));
-                    } else {
-                        const float sdf_n = fminf(fmaxf(__fmul_rn(sd[j], v.inv_trunc), -1.0f), 1.0f);
-                        fix = to_fix(sdf_n);
-                        // Kept for the records of voxels that cross the cap, so the
-                        // update tail never reads the batch's points again.
-                        store_slot(u.slot_val + (rec - u.records), sdf_n);
-                    }
-                    red_add(&u.vcnt[out], 1u);
-                    red_add(&u.vacc[out], (unsigned long long)fix);
-                    ++counted;
-                }
-                if (i < a.n) store_slot(rec, out);  // read again by the group pass
-                rec += a.n;
+                const float t = __fmul_rn((float)c0 + (float)j, v.voxel_size);
+                const float yx = __fadd_rd(__fmul_rn(__fadd_rn(px, __fmul_rn(r.ux, t)), v.inv_voxel), kFloorMagic);
+                const float yy = __fadd_rd(__fmul_rn(__fadd_rn(py, __fmul_rn(r.uy, t)), v.inv_voxel), kFloorMagic);
+                const float yz = __fadd_rd(__fmul_rn(__fadd_rn(pz, __fmul_rn(r.uz, t)), v.inv_voxel), kFloorMagic);
+                const float ex = __fsub_rn(__fmaf_rn(__fsub_rn(yx, kFloorMagic), v.voxel_size, half), cx);
+                const float ey = __fsub_rn(__fmaf_rn(__fsub_rn(yy, kFloorMagic), v.voxel_size, half), cy);
+                const float ez = __fsub_rn(__fmaf_rn(__fsub_rn(yz, kFloorMagic), v.voxel_size, half), cz);
+                dsq[j] = __fadd_rn(__fadd_rn(__fmul_rn(ex, ex), __fmul_rn(ey, ey)), __fmul_rn(ez, ez));
+                const uint32_t w = pack_offset(__float_as_uint(yx), __float_as_uint(yy), __float_as_uint(yz)) - base;
+                bool ok = mine && j < n_steps;
+                if (c0 + j > sure_step) ok = ok && !(__fsub_rn(r.dist, __fsqrt_rn(dsq[j])) < -v.trunc);
+                vox[j] = ok ? w : kNoOffset;
+                if (ok) table[table_entry(w)].x = w & kOffsetBlock;
             }
+            __syncwarp();
+
+            bool met = false;
+            unsigned done = 0u;  // once met: bit j, sample j has its voxel
+            for (;;) {
+                // The blocks in the table, one or two per lane. A slot's 16
+                // bytes hold the key, the index and the touch tag.
+                bool dropped = false;
+#pragma unroll
+                for (int k = 0; k < kTableEntries / 32; ++k) {
+                    const uint32_t b = table[lane + 32 * k].x;
+                    const bool need = b != kNoOffset;
+                    if (k > 0 && !__any_sync(0xffffffffu, need)) break;
+                    const uint32_t kx = (uint32_t)((int)(ox - kFloorBits) >> 3) + (uint32_t)kCoordBias + ((b >> 3) & 255u);
+                    const uint32_t ky = (uint32_t)((int)(oy - kFloorBits) >> 3) + (uint32_t)kCoordBias + ((b >> 14) & 255u);
+                    const uint32_t kz = (uint32_t)((int)(oz - kFloorBits) >> 3) + (uint32_t)kCoordBias + (b >> 25);
+                    const uint2 key = make_uint2(kz | ky << kCoordBits, ky >> (32 - kCoordBits) | kx << (2 * kCoordBits - 32));
+                    Resolved res{-1, home_slot(v, key)};
+                    bool rest = false;
+                    uint32_t seen = 0u;
+                    if (need) {
+                        seen = probe_settle<MODE>(v, probe_start<MODE>(v, res.slot), key, res);
+                        rest = res.bi == kUnsettled;
+                    }
+                    // The lanes' keys are distinct: each probes for itself.
+                    if (rest) res = resolve<MODE>(v, (long long)((unsigned long long)key.y << 32 | key.x), nullptr, 0);
+                    __syncwarp();
+                    if (RECORDS) tag_touched<false>(v, u, res.bi >= 0 && (rest || seen != u.tag), res.bi, res.slot);
+                    if (need) table[lane + 32 * k].y = (uint32_t)res.bi;
+                    dropped |= need && res.bi < 0;
+                }
+                __syncwarp();
+                if (!met) {
+                    // Every sample's entry, all loads in flight together, no branch.
+                    bool miss = false;
+                    uint32_t at[kChunk];
+#pragma unroll
+                    for (int j = 0; j < kChunk; ++j) {
+                        const uint2 e = table[table_entry(vox[j])];
+                        const bool hit = e.x == (vox[j] & kOffsetBlock);
+                        miss |= !hit && vox[j] != kNoOffset;
+                        at[j] = hit ? __funnelshift_l(voxel_high(vox[j]), e.y, 9) : kNoVoxel;
+                        // The oracle's value needs the voxel's offset.
+                        if constexpr (S == kStoreF64) dsq[j] = __uint_as_float(vox[j]);
+                    }
+                    if (!__any_sync(0xffffffffu, miss || dropped)) {
+#pragma unroll
+                        for (int j = 0; j < kChunk; ++j) vox[j] = at[j];
+                        break;
+                    }
+                }
+                // Two blocks met in an entry (met: further rounds for the
+                // samples left), or a block was dropped.
+                met = true;
+                bool left = false;
+#pragma unroll
+                for (int j = 0; j < kChunk; ++j) {
+                    if (vox[j] == kNoOffset || ((done >> j) & 1u)) continue;
+                    const uint2 e = table[table_entry(vox[j])];
+                    if (e.x != (vox[j] & kOffsetBlock)) {
+                        left = true;
+                        continue;
+                    }
+                    done |= 1u << j;
+                    if (counts_drops && (int)e.y < 0) ++drops;
+                    vox[j] = (int)e.y < 0 ? kNoVoxel : __funnelshift_l(voxel_high(vox[j]), e.y, 9);
+                }
+                if (!__any_sync(0xffffffffu, left)) break;
+                __syncwarp();
+                table[lane].x = kNoOffset;
+                table[lane + 32].x = kNoOffset;
+                __syncwarp();
+#pragma unroll
+                for (int j = 0; j < kChunk; ++j)
+                    if (vox[j] != kNoOffset && !((done >> j) & 1u)) table[table_entry(vox[j])].x = vox[j] & kOffsetBlock;
+                __syncwarp();
+            }
+            if (RECORDS)
+                count_samples<S>(v, u, writes, (uint32_t)a.n, r.dist, vox, dsq, n_steps, slot, counted, [&](int j) {
+                    const uint32_t w = __float_as_uint(dsq[j]);
+                    return oracle_fix(v, a, r, (int)(ox - kFloorBits + (w & 2047u)),
+                                      (int)(oy - kFloorBits + ((w >> 11) & 2047u)), (int)(oz - kFloorBits + (w >> 22)));
+                });
+            __syncwarp();  // the table is rewritten by the next chunk
         }
-        __syncwarp();  // run columns are rewritten by the next chunk
+        todo &= ~group;
+    }
+
+    // Points far apart or far away: one sample at a time.
+    if (todo == 0u) return;
+    const bool mine = (todo >> lane) & 1u;
+    uint32_t slot = (uint32_t)i;
+    Resolved res{-1, 0u};
+    int ox = 0, oy = 0, oz = 0;
+    bool started = false;
+#pragma unroll 1
+    for (int s = -v.steps; s <= v.steps; ++s) {
+        int vx = 0, vy = 0, vz = 0;
+        float dsq[1] = {0.0f};
+        const bool ok = mine && band_sample_ray(v, r, s, vx, vy, vz, dsq[0]);
+        // A straight ray leaves a block (a convex box) for good, so equal
+        // consecutive blocks are the only repeats.
+        const bool fresh = ok && (!started || (((vx ^ ox) | (vy ^ oy) | (vz ^ oz)) >> 3) != 0);
+        const unsigned long long k = (unsigned long long)pack_key(vx >> 3, vy >> 3, vz >> 3);
+        bool rest = false, old = false;
+        if (fresh) {
+            const uint2 key = make_uint2((uint32_t)k, (uint32_t)(k >> 32));
+            res.slot = home_slot(v, key);
+            old = probe_settle<MODE>(v, probe_start<MODE>(v, res.slot), key, res) != u.tag;
+            rest = res.bi == kUnsettled;
+            started = true;
+            ox = vx;
+            oy = vy;
+            oz = vz;
+        }
+        resolve_grouped<MODE>(v, rest, (long long)k, res, hist, n_bins);
+        if (RECORDS) tag_touched<true>(v, u, fresh && res.bi >= 0 && (rest || old), res.bi, res.slot);
+        uint32_t vox[1] = {kNoVoxel};
+        if (ok && res.bi >= 0)
+            vox[0] = (uint32_t)res.bi * kBlockVoxels + (uint32_t)(((vz & 7) * kBlockDim + (vy & 7)) * kBlockDim + (vx & 7));
+        if (counts_drops && ok && res.bi < 0) ++drops;
+        if (RECORDS)
+            count_samples<S>(v, u, mine || (round == 0 && in_batch && !live), (uint32_t)a.n, r.dist, vox, dsq, 1, slot, counted,
+                             [&](int) { return oracle_fix(v, a, r, vx, vy, vz); });
     }
 }
 
@@ -417,7 +642,7 @@ template <int MODE, bool RECORDS, int S, bool FRAMES, typename Points, typename 
 __device__ __forceinline__ void band_tiles(const DevVolume& v, const BatchArgs& a, const UpdateScratch& u,
                                            unsigned long long* hist, int n_bins, const Points pts,
                                            Camera cam) {
-    __shared__ BandSmem sm;
+    __shared__ BandSmem<!has_fast_probe<MODE>()> sm;
     const int t = threadIdx.x;
     const int lane = t & 31;
     const bool counts_drops = MODE != kLookupOnly && MODE != kAllocNoCas && MODE != kAllocCountingCas;
@@ -446,7 +671,7 @@ __device__ __forceinline__ void band_tiles(const DevVolume& v, const BatchArgs& 
         nhas = false;
         if (inext < a.n) nhas = pts.load(inext, nx, ny, nz);
         cam.at(i);
-        band_point<MODE, RECORDS, S, kProbeWarp, FRAMES>(v, a, u, i, has, px, py, pz, sm, drops, counted,
+        band_point<MODE, RECORDS, S, FRAMES>(v, a, u, i, has, px, py, pz, sm, drops, counted,
                                                          hist, n_bins, cam.cx, cam.cy, cam.cz);
     }
 
@@ -469,7 +694,7 @@ band_kernel(DevVolume v, BatchArgs a, UpdateScratch u, unsigned long long* hist,
 // Integrate (allocate + count-and-sum) of a batch of several frames: the
 // single-frame walk with each point's camera taken from the frame table.
 template <int S>
-__global__ void __launch_bounds__(kBandThreads, kBandFramesMinBlocks)
+__global__ void __launch_bounds__(kBandThreads, kBandMinBlocks)
 band_frames_kernel(DevVolume v, BatchArgs a, UpdateScratch u, const FrameCam* frames, int32_t n_frames) {
     if (OSN_BAND_PDL) grid_dependency_wait();  // the set-up kernel's frame table and zeroed counters
     band_tiles<kAllocInsert, true, S, true>(v, a, u, nullptr, 0, BatchPoints<0>{a}, FrameCursor(frames, n_frames));
@@ -478,7 +703,7 @@ band_frames_kernel(DevVolume v, BatchArgs a, UpdateScratch u, const FrameCam* fr
 // The same for several depth images of equal size: each CTA stages the
 // images' poses in shared memory first.
 template <int S>
-__global__ void __launch_bounds__(kBandThreads, kBandFramesMinBlocks)
+__global__ void __launch_bounds__(kBandThreads, kBandMinBlocks)
 band_depth_frames_kernel(DevVolume v, BatchArgs a, UpdateScratch u, const FrameCam* frames,
                          const FramePose* poses, int32_t n_frames) {
     __shared__ FramePose s_pose[kMaxDepthFrames];
@@ -547,10 +772,10 @@ __device__ __forceinline__ int scene_of(const int* begin, int n, int item) {
 // out by an atomic queue to a persistent grid; the CTA keeps the current
 // item's scene descriptor in shared memory and flushes its per-scene
 // counters whenever it moves to another scene.
-template <int S, int PROBE>
-__global__ void __launch_bounds__(kBandThreads, kBandFramesMinBlocks)
+template <int S>
+__global__ void __launch_bounds__(kBandThreads, kBandMinBlocks)
 band_multi_kernel(StepWork w) {
-    __shared__ BandSmem sm;
+    __shared__ BandSmem<false> sm;
     __shared__ SceneWork sw;
     __shared__ int s_begin[kMaxBatchScenes + 1];
     __shared__ int s_item;
@@ -607,7 +832,7 @@ band_multi_kernel(StepWork w) {
             const int i = tile * kBandThreads + t;
             float px = 0.0f, py = 0.0f, pz = 0.0f;
             const bool has = i < sw.a.n && load_point(sw.a, i, px, py, pz);
-            band_point<kAllocInsert, true, S, PROBE>(sw.v, sw.a, sw.u, i, has, px, py, pz, sm, drops,
+            band_point<kAllocInsert, true, S>(sw.v, sw.a, sw.u, i, has, px, py, pz, sm, drops,
                                                     counted, nullptr, 0);
         }
         __syncthreads();  // s_item and the descriptor are rewritten next
@@ -751,32 +976,25 @@ cudaError_t launch_band_frames(const DevVolume& v, const BatchArgs& a, const Upd
 }
 
 namespace {
-template <int S, int PROBE>
+template <int S>
 cudaError_t launch_band_multi_t(const StepWork& w, int sm_count, cudaStream_t s) {
     static int per_sm = 0;
     static std::once_flag once;
     std::call_once(once, [] {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, band_multi_kernel<S, PROBE>,
-                                                          kBandThreads, 0) != cudaSuccess ||
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, band_multi_kernel<S>, kBandThreads, 0) !=
+                cudaSuccess ||
             per_sm < 1)
             per_sm = 1;
     });
-    return launch_after(band_multi_kernel<S, PROBE>, per_sm * sm_count, kBandThreads, s, w);
+    return launch_after(band_multi_kernel<S>, per_sm * sm_count, kBandThreads, s, w);
 }
 }  // namespace
 
-cudaError_t launch_band_multi(const StepWork& w, int storage, int probe, int sm_count, cudaStream_t s) {
-    const bool lane = probe == kProbeLane;
+cudaError_t launch_band_multi(const StepWork& w, int storage, int sm_count, cudaStream_t s) {
     switch (storage) {
-        case kStoreF16U16:
-            return lane ? launch_band_multi_t<kStoreF16U16, kProbeLane>(w, sm_count, s)
-                        : launch_band_multi_t<kStoreF16U16, kProbeWarp>(w, sm_count, s);
-        case kStoreF64:
-            return lane ? launch_band_multi_t<kStoreF64, kProbeLane>(w, sm_count, s)
-                        : launch_band_multi_t<kStoreF64, kProbeWarp>(w, sm_count, s);
-        default:
-            return lane ? launch_band_multi_t<kStoreF32, kProbeLane>(w, sm_count, s)
-                        : launch_band_multi_t<kStoreF32, kProbeWarp>(w, sm_count, s);
+        case kStoreF16U16: return launch_band_multi_t<kStoreF16U16>(w, sm_count, s);
+        case kStoreF64: return launch_band_multi_t<kStoreF64>(w, sm_count, s);
+        default: return launch_band_multi_t<kStoreF32>(w, sm_count, s);
     }
 }
 

@@ -67,7 +67,7 @@ constexpr float kU16WeightMax = 65535.0f;
 struct HashEntry {
     long long key;
     int32_t block_idx;
-    int32_t pad;
+    int32_t pad;  // the update that last touched the block (0: none since the table was filled)
 };
 static_assert(sizeof(HashEntry) == 16, "hash slot must stay 16 bytes");
 
@@ -94,6 +94,7 @@ struct DevVolume {
     float inv_trunc;  // 1.0f / trunc (volume.cpp:203)
     float weight_cap;  // effective cap: <= 0 disables (FP32/FP64); at most 65535 for uint16 weights
     int32_t steps;    // max(1, ceil(trunc * inv_voxel)) (volume.cpp:171)
+    int32_t sure_step;  // the last band step a whole voxel short of the truncation distance
     uint32_t* status;
     int32_t storage;     // Storage
     int32_t spin_limit;  // iterations a publication wait may take (kSpinLimit by default)
@@ -279,7 +280,8 @@ __device__ __forceinline__ bool ray_setup(const BatchArgs& a, int i, Ray& r) {
 // voxel CENTRE. False when the voxel is fully occluded (sdf < -trunc), the
 // gate both passes apply (volume.cpp:185-191, :260-268).
 __device__ __forceinline__ bool band_sample_from(const DevVolume& v, const Ray& r, float cx, float cy,
-                                                 float cz, int s, int& vx, int& vy, int& vz, float& sdf) {
+                                                 float cz, int s, int& vx, int& vy, int& vz, float& sdf,
+                                                 float& dsq) {
     const float t = __fmul_rn((float)s, v.voxel_size);
     vx = (int)floorf(__fmul_rn(__fadd_rn(r.px, __fmul_rn(r.ux, t)), v.inv_voxel));
     vy = (int)floorf(__fmul_rn(__fadd_rn(r.py, __fmul_rn(r.uy, t)), v.inv_voxel));
@@ -287,22 +289,24 @@ __device__ __forceinline__ bool band_sample_from(const DevVolume& v, const Ray& 
     const float ex = __fsub_rn(__fmul_rn(__fadd_rn((float)vx, 0.5f), v.voxel_size), cx);
     const float ey = __fsub_rn(__fmul_rn(__fadd_rn((float)vy, 0.5f), v.voxel_size), cy);
     const float ez = __fsub_rn(__fmul_rn(__fadd_rn((float)vz, 0.5f), v.voxel_size), cz);
-    const float dv =
-        __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(ex, ex), __fmul_rn(ey, ey)), __fmul_rn(ez, ez)));
-    sdf = __fsub_rn(r.dist, dv);
+    dsq = __fadd_rn(__fadd_rn(__fmul_rn(ex, ex), __fmul_rn(ey, ey)), __fmul_rn(ez, ez));
+    sdf = __fsub_rn(r.dist, __fsqrt_rn(dsq));
     return !(sdf < -v.trunc);
 }
 
 // A batch with one camera (read from the batch's arguments).
 __device__ __forceinline__ bool band_sample(const DevVolume& v, const BatchArgs& a, const Ray& r,
                                             int s, int& vx, int& vy, int& vz, float& sdf) {
-    return band_sample_from(v, r, a.cam_x, a.cam_y, a.cam_z, s, vx, vy, vz, sdf);
+    float dsq;
+    return band_sample_from(v, r, a.cam_x, a.cam_y, a.cam_z, s, vx, vy, vz, sdf, dsq);
 }
 
-// A batch of several frames: the camera of the point's frame, kept in the ray.
+// The same with the camera of the point's frame, kept in the ray; gives the
+// squared distance of camera and voxel centre in place of the signed distance.
 __device__ __forceinline__ bool band_sample_ray(const DevVolume& v, const Ray& r, int s, int& vx,
-                                                int& vy, int& vz, float& sdf) {
-    return band_sample_from(v, r, r.cx, r.cy, r.cz, s, vx, vy, vz, sdf);
+                                                int& vy, int& vz, float& dsq) {
+    float sdf;
+    return band_sample_from(v, r, r.cx, r.cy, r.cz, s, vx, vy, vz, sdf, dsq);
 }
 
 // The FP64 oracle's signed distance of the same band sample: the point's
@@ -325,20 +329,28 @@ __device__ __forceinline__ double clamp_sdf_n_f64(double sdf, float trunc) {
 
 // ---- lookups after allocation has completed --------------------------------
 
-// Block index of a key, or -1 (volume.cpp:71-92). Only valid in kernels that
-// run after the allocating kernel finished, so every index is published and
-// the non-coherent 128-bit load of a whole slot is safe.
+// Block index of a key, or -1 (volume.cpp:71-92), and how many slots were
+// visited (the last one holds the key when the index is valid). Only valid in
+// kernels that run after the allocating kernel finished, so every index is
+// published; slots are read through L1, where a concurrent update may leave
+// only their touch tag (pad) out of date.
 __device__ __forceinline__ int32_t find_block(const DevVolume& v, int32_t bx, int32_t by, int32_t bz,
-                                              long long want) {
+                                              long long want, uint32_t& probes) {
     const uint32_t size = v.hash_mask + 1;
     const uint32_t start = hash_slot(bx, by, bz, v.hash_mask);
     for (uint32_t p = 0; p < size; ++p) {
-        const int4 raw = __ldg(reinterpret_cast<const int4*>(&v.table[(start + p) & v.hash_mask]));
+        probes = p + 1;
+        const int4 raw = __ldca(reinterpret_cast<const int4*>(&v.table[(start + p) & v.hash_mask]));
         const long long key = ((long long)(unsigned)raw.y << 32) | (unsigned)raw.x;
         if (key == want) return (raw.z >= 0 && raw.z < v.pool_capacity) ? raw.z : -1;
         if (key == kEmptyKey) return -1;
     }
     return -1;
+}
+__device__ __forceinline__ int32_t find_block(const DevVolume& v, int32_t bx, int32_t by, int32_t bz,
+                                              long long want) {
+    uint32_t probes;
+    return find_block(v, bx, by, bz, want, probes);
 }
 
 // ---- insertion (volume.cpp:94-145, volume_cuda.cu:59-107) -------------------
@@ -356,7 +368,7 @@ enum AllocMode : int {
 
 struct InsertResult {
     int32_t idx;      // >= 0 allocated or found, -1 dropped / absent
-    uint32_t probes;  // slots visited
+    uint32_t probes;  // slots visited: the last of them is home slot + probes - 1
 };
 
 // Wait, with an iteration bound, until a claimed slot's index is published

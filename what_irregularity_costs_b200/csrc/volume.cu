@@ -64,6 +64,8 @@ Volume::Volume(float voxel, int32_t pool, float trunc_m, float weight_cap, uint3
     weight_cap_ = weight_cap;
     dv_.pool_capacity = pool;
     dv_.steps = std::max(1, (int32_t)std::ceil(dv_.trunc * dv_.inv_voxel));
+    dv_.sure_step = -dv_.steps - 1;
+    while (dv_.sure_step < dv_.steps && (float)(dv_.sure_step + 2) * voxel <= dv_.trunc) ++dv_.sure_step;
     dv_.spin_limit = kSpinLimit;
     ok_ = alloc_device(hash_slots);
 }
@@ -97,7 +99,6 @@ bool Volume::alloc_device(uint32_t hash_slots) {
     }
     OSN_TRY(cudaMalloc(&us_.vcnt, n_vox * sizeof(uint32_t)));
     OSN_TRY(cudaMalloc(&us_.vacc, n_vox * sizeof(unsigned long long)));
-    OSN_TRY(cudaMalloc(&us_.blk_touch, (size_t)dv_.pool_capacity * sizeof(uint32_t)));
     OSN_TRY(cudaMalloc(&us_.xbits, (size_t)dv_.pool_capacity * kXWords * sizeof(uint32_t)));
     OSN_TRY(cudaMalloc(&us_.touched, (size_t)dv_.pool_capacity * sizeof(int32_t)));
     OSN_TRY(cudaMalloc(&us_.ctl, sizeof(UpdateControl)));
@@ -124,7 +125,6 @@ bool Volume::alloc_device(uint32_t hash_slots) {
     }
     OSN_TRY(cudaMemsetAsync(us_.vcnt, 0, n_vox * sizeof(uint32_t), stream_));
     OSN_TRY(cudaMemsetAsync(us_.vacc, 0, n_vox * sizeof(unsigned long long), stream_));
-    OSN_TRY(cudaMemsetAsync(us_.blk_touch, 0, (size_t)dv_.pool_capacity * sizeof(uint32_t), stream_));
     OSN_TRY(cudaMemsetAsync(us_.xbits, 0, (size_t)dv_.pool_capacity * kXWords * sizeof(uint32_t), stream_));
     OSN_TRY(cudaMemsetAsync(us_.ctl, 0, sizeof(UpdateControl), stream_));
     OSN_TRY(cudaStreamSynchronize(stream_));
@@ -145,7 +145,6 @@ Volume::~Volume() {
     cudaFree(dv_.b);
     cudaFree(us_.vcnt);
     cudaFree(us_.vacc);
-    cudaFree(us_.blk_touch);
     cudaFree(us_.xbits);
     cudaFree(us_.touched);
     cudaFree(us_.ctl);
@@ -341,7 +340,7 @@ cudaError_t Volume::run_update(const BatchArgs& a, const UpdateScratch& scratch,
     // Block tags are update numbers; at the (theoretical) wrap, clear them.
     if (++update_tag_ == 0u) {
         join();
-        cudaMemsetAsync(us_.blk_touch, 0, (size_t)dv_.pool_capacity * sizeof(uint32_t), stream_);
+        cudaMemset2DAsync(&dv_.table->pad, sizeof(HashEntry), 0, sizeof(int32_t), (size_t)dv_.hash_mask + 1, stream_);
         update_tag_ = 1u;
     }
     UpdateScratch u = scratch;
@@ -496,7 +495,7 @@ bool Volume::reserve_batch(int32_t max_points) {
 SceneWork Volume::batch_work(const BatchArgs& a, cudaStream_t s) {
     // Block tags are update numbers; at the (theoretical) wrap, clear them.
     if (++update_tag_ == 0u) {
-        cudaMemsetAsync(us_.blk_touch, 0, (size_t)dv_.pool_capacity * sizeof(uint32_t), s);
+        cudaMemset2DAsync(&dv_.table->pad, sizeof(HashEntry), 0, sizeof(int32_t), (size_t)dv_.hash_mask + 1, s);
         update_tag_ = 1u;
     }
     SceneWork w{};

@@ -96,14 +96,14 @@ struct UpdateScratch {
                                          // records still to be placed in its group)
     unsigned long long* vacc = nullptr;  // fixed-point sum of their sdf_n (of a crossing voxel: group
                                          // base + 1 << 32 | next place)
-    // Per block, tagged with the update number instead of being cleared.
-    uint32_t* blk_touch = nullptr;  // update that last touched the block
     // [pool * kXWords] per block: bit lv set when voxel lv crosses the cap in
     // this update; rewritten by finish for every block whose voxels it reads.
     uint32_t* xbits = nullptr;
     int32_t* touched = nullptr;     // [pool] blocks touched by this update
     uint32_t* status = nullptr;     // the volume's status word
-    uint32_t tag = 0;               // this update's number (never 0)
+    // This update's number (never 0): the spare word of a touched block's
+    // table slot holds it, instead of a flag that would have to be cleared.
+    uint32_t tag = 0;
 };
 
 // A volume's counters, one allocation (a reset clears them together).
@@ -362,7 +362,7 @@ enum BatchQueue : int { kQBand = 0, kQFinish, kQGroup, kQSelect, kNumBatchQueues
 // Tunable shape of a batched step (chosen by the batch autotuner).
 struct BatchShape {
     int band_tiles_per_item = 4;  // band work item: this many 128-point tiles of one scene
-    int probe = 0;                // 0: warp-deduplicated block resolution, 1: per-lane
+    int probe = 0;                // accepted (0 or 1); the walk has one resolution scheme now
     int finish_pair = 1;          // finish work item: 1 = two touched blocks, 0 = one
 };
 
@@ -376,7 +376,7 @@ struct StepWork {
 };
 
 cudaError_t launch_batch_prepare(const StepWork& w, cudaStream_t s);
-cudaError_t launch_band_multi(const StepWork& w, int storage, int probe, int sm_count, cudaStream_t s);
+cudaError_t launch_band_multi(const StepWork& w, int storage, int sm_count, cudaStream_t s);
 cudaError_t launch_finish_multi(const StepWork& w, int storage, int pair, int sm_count, cudaStream_t s);
 cudaError_t launch_group_multi(const StepWork& w, int storage, int sm_count, cudaStream_t s);
 cudaError_t launch_select_multi(const StepWork& w, int storage, int sm_count, cudaStream_t s);
