@@ -80,3 +80,19 @@ def test_walk_drops_where_the_pool_is_full(cuda):
     for c, w in zip(coords.tolist(), weight):
         assert np.array_equal(w, want[tuple(c)])
     assert vol.drop_count() == int(rw.sum() - weight.sum())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 7, 29, 257, 2051])
+@pytest.mark.parametrize("cap", [1.0, 5.0])
+def test_every_record_crosses(cuda, n, cap):
+    """Grouping where all 256 band slots of a warp belong to cap-crossing
+    voxels, and where the slots end inside a thread's eight."""
+    points = np.tile(np.array([[0.013, 0.021, 1.007]], dtype=np.float32), (n, 1))
+    points[1::3, 0] += np.float32(0.3)
+    vol = CudaVolume(0.02, 1 << 10, 0.08, cap)
+    ref = oracle.OracleVolume(0.02, 1 << 10, 0.08, cap)
+    vol.integrate(cuda.from_numpy(points).cuda(), (0.0, 0.0, 0.0))
+    ref.integrate(points, (0.0, 0.0, 0.0))
+    assert vol.status() == 0
+    assert_same_voxels(vol, ref)

@@ -31,17 +31,16 @@
 //            crossing bitmap (16 words per block, rewritten for every block
 //            finish visits).
 //   group    one pass over the band slots of the batch, eight per thread
-//            (records loaded as 128-bit vectors): a record whose voxel's bit
-//            is set takes the next place of the voxel's group (atomic add on
-//            the sum word; its normalised SDF loaded in the same round trip)
-//            and stores its canonical id and value there, then counts the
-//            voxel's pending
-//            records down with an acquire-release atomic. The record that
-//            brings the count to zero is the last of its group: its warp
-//            loads the whole group, keeps the keep records with the smallest
-//            ids (shuffle ranking in registers up to 256 records, a radix
-//            select beyond) and finishes the voxel. No pass runs between the
-//            grouping and the selection.
+//            (records loaded as 128-bit vectors): the records of voxels whose
+//            bit is set are packed across the warp, and each takes the next
+//            place of its voxel's group (atomic add on the sum word; its
+//            normalised SDF loaded in the same round trip) and stores its
+//            canonical id and value there.
+//   select   over the list of crossing voxels: the keep records with the
+//            smallest ids of each group are summed (shuffle ranking in
+//            registers up to 256 records, a radix select beyond) and the voxel
+//            is finished. A pass of its own, so the pass boundary orders the
+//            group's entries.
 //
 // The FP64 oracle storage keeps no per-slot values: its group entries hold
 // the band slot, and the selection recomputes each record's normalised SDF
@@ -64,19 +63,6 @@ constexpr int kGroupThreads = 256;
 constexpr int kGroupWarps = kGroupThreads / 32;
 constexpr int kGroupPerThread = 8;  // band slots per thread (two 128-bit loads)
 constexpr int kRankRegs = 8;        // groups of up to 32 * 8 records are ranked in registers
-// Where the ordered selection of cap-crossing voxels runs: 1, in its own
-// pass over a list of the crossing voxels that finish writes (no memory
-// ordering inside a pass: the pass boundary orders everything); 0, inside
-// the group pass, by the warp whose record completes a voxel's group (one
-// fence per thread that placed records, one per selected group).
-#ifndef OSN_SPLIT_SELECT
-#define OSN_SPLIT_SELECT 1
-#endif
-// The group pass as a persistent grid whose threads load their next chunk of
-// records before placing the current one (1), or one chunk per thread (0).
-#ifndef OSN_GROUP_PERSISTENT
-#define OSN_GROUP_PERSISTENT 0
-#endif
 constexpr int kSelectThreads = 128;
 constexpr int kSelectWarps = kSelectThreads / 32;
 // Resident 256-thread CTAs per SM the group pass's registers are sized for:
@@ -259,7 +245,7 @@ __device__ __forceinline__ void finish_quad(const DevVolume& v, const UpdateScra
                 acc[q] = (unsigned long long)(rec_base + 1u) << 32;
                 cnt[q] = n[q];
                 xmask |= 1u << q;
-                if (OSN_SPLIT_SELECT) u.xlist[x_at] = (uint32_t)bi * kBlockVoxels + 4u * t + q;
+                u.xlist[x_at] = (uint32_t)bi * kBlockVoxels + 4u * t + q;
             } else {
                 // Out of scratch (only after a failed update left stale
                 // counters): the voxel's records are dropped, the status
@@ -555,11 +541,6 @@ __device__ __forceinline__ long long large_group_sum(const DevVolume& v, const B
 template <int S>
 __device__ __forceinline__ int select_group(const SelectArgs& sa, const DevVolume& v, const BatchArgs& a,
                                             uint32_t vi, uint32_t* hist, int lane) {
-    // Fused selection: the group's other records were placed by other
-    // threads of this pass, each with a fence between its entry stores and
-    // its countdown; this fence orders the reads below after the countdown
-    // that saw the group complete.
-    if (!OSN_SPLIT_SELECT) __threadfence();
     const unsigned long long h = __ldcg(&sa.vacc[vi]);
     const uint32_t base = (uint32_t)(h >> 32) - 1u;
     const int n = (int)(uint32_t)h;
@@ -579,19 +560,6 @@ __device__ __forceinline__ int select_group(const SelectArgs& sa, const DevVolum
     return 1;
 }
 
-// The same out of line for the storages whose entries carry their values
-// (no volume or batch needed): the selection runs about once per warp, so
-// the scan of the band slots keeps its few registers and its occupancy.
-template <int S>
-__device__ __noinline__ int select_group_out(const SelectArgs sa, uint32_t vi, uint32_t* hist, int lane) {
-    static_assert(S != kStoreF64, "the FP64 oracle recomputes values from its batch");
-    return select_group<S>(sa, DevVolume{}, BatchArgs{}, vi, hist, lane);
-}
-
-// Eight band slots from `first` of one batch, by every thread of the warp
-// (warp-synchronous): records of voxels whose crossing bit is set take their
-// place in the voxel's group; the warp then selects and finishes every group
-// one of its records completed.
 // The records of eight band slots from `first` (kNoVoxel past the batch).
 __device__ __forceinline__ void load_records(const UpdateScratch& u, uint32_t first, uint32_t n_slots,
                                              uint32_t (&vi)[kGroupPerThread]) {
@@ -608,12 +576,9 @@ __device__ __forceinline__ void load_records(const UpdateScratch& u, uint32_t fi
     }
 }
 
-// Records of voxels whose crossing bit is set take their place in the
-// voxel's group; returns bit m set for slot m placed.
-template <int S>
-__device__ __forceinline__ uint32_t place_records(const BatchArgs& a, const DevVolume& v, const UpdateScratch& u,
-                                                  uint32_t first, const uint32_t (&vi)[kGroupPerThread]) {
-    // Crossing bits: one gather per distinct bitmap word among the eight.
+// Bit m set: slot m's voxel crosses the cap in this update. One bitmap gather
+// per distinct word among the eight.
+__device__ __forceinline__ uint32_t crossing_slots(const UpdateScratch& u, const uint32_t (&vi)[kGroupPerThread]) {
     uint32_t word[kGroupPerThread];
     bool same[kGroupPerThread];
 #pragma unroll
@@ -621,70 +586,57 @@ __device__ __forceinline__ uint32_t place_records(const BatchArgs& a, const DevV
         same[m] = m > 0 && vi[m] != kNoVoxel && vi[m - 1] != kNoVoxel && (vi[m - 1] >> 5) == (vi[m] >> 5);
         word[m] = (vi[m] == kNoVoxel || same[m]) ? 0u : __ldg(&u.xbits[vi[m] >> 5]);
     }
-#pragma unroll
-    for (int m = 1; m < kGroupPerThread; ++m)
-        if (same[m]) word[m] = word[m - 1];
-    const uint32_t n_steps = 2u * (uint32_t)v.steps + 1u;
-    uint32_t placed = 0u;  // bit m: slot m's record took a place in its group
+    uint32_t cross = 0u;
 #pragma unroll
     for (int m = 0; m < kGroupPerThread; ++m) {
-        if (vi[m] == kNoVoxel || !((word[m] >> (vi[m] & 31u)) & 1u)) continue;
-        const uint32_t slot = first + m;
-        // The record's value (FP32 / FP16: the walk kept it) is loaded beside
-        // its place ticket, in the same round trip.
-        float val = 0.0f;
-        if constexpr (S != kStoreF64) val = __ldcs(u.slot_val + slot);
-        const unsigned long long tk = atomicAdd(&u.vacc[vi[m]], 1ull);
-        const uint64_t pos = (uint64_t)((uint32_t)(tk >> 32) - 1u) + (uint32_t)tk;
-        unsigned long long e;
-        if constexpr (S == kStoreF64)
-            e = slot;
-        else
-            e = (unsigned long long)slot_id(slot, (uint32_t)a.n, n_steps) |
-                ((unsigned long long)__float_as_uint(val) << 32);
-        if (pos < (uint64_t)u.record_cap) u.grp[pos] = e;
-        else atomicOr(u.status, kStatusScratchOverflow);  // state left by a failed update
-        placed |= 1u << m;
+        if (m > 0 && same[m]) word[m] = word[m - 1];
+        cross |= ((word[m] >> (vi[m] & 31u)) & 1u) << m;
     }
-    return placed;
+    return cross;
 }
 
+// One record of a cap-crossing voxel takes the next place of the voxel's group.
 template <int S>
-__device__ __forceinline__ void group_slots(const DevVolume& v, const BatchArgs& a, const UpdateScratch& u,
-                                            uint32_t first, uint32_t n_slots, uint32_t* hist, int& updated) {
+__device__ __forceinline__ void place_record(const DevVolume& v, const BatchArgs& a, const UpdateScratch& u,
+                                             uint32_t slot, uint32_t vi) {
+    // The record's value (FP32 / FP16: the walk kept it) is loaded beside its
+    // place ticket, in the same round trip.
+    const unsigned long long tk = atomicAdd(&u.vacc[vi], 1ull);
+    float val = 0.0f;
+    if constexpr (S != kStoreF64) val = __ldcs(u.slot_val + slot);
+    const uint64_t pos = (uint64_t)((uint32_t)(tk >> 32) - 1u) + (uint32_t)tk;
+    unsigned long long e;
+    if constexpr (S == kStoreF64)
+        e = slot;
+    else
+        e = (unsigned long long)slot_id(slot, (uint32_t)a.n, 2u * (uint32_t)v.steps + 1u) |
+            ((unsigned long long)__float_as_uint(val) << 32);
+    if (pos < (uint64_t)u.record_cap) u.grp[pos] = e;
+    else atomicOr(u.status, kStatusScratchOverflow);  // state left by a failed update
+}
+
+// The crossing records among eight slots per lane, placed by the whole warp:
+// about one slot in ten crosses, so they are first packed into the warp's
+// queue (slot, voxel) and then taken 32 at a time. Placing them where they
+// were found ran eight nearly empty passes over a warp, each with its own
+// round trip (36 us on four 640x480 frames; 30 packed).
+template <int S>
+__device__ __forceinline__ void place_records(const BatchArgs& a, const DevVolume& v, const UpdateScratch& u,
+                                              uint32_t first, const uint32_t (&vi)[kGroupPerThread], uint2* queue) {
+    const uint32_t cross = crossing_slots(u, vi);
+    if (!__any_sync(0xffffffffu, cross != 0u)) return;
     const int lane = threadIdx.x & 31;
-    uint32_t vi[kGroupPerThread];
-    load_records(u, first, n_slots, vi);
-    const uint32_t placed = place_records<S>(a, v, u, first, vi);
-    if (OSN_SPLIT_SELECT) return;  // the select pass ranks the complete groups
-    // Fused selection: this thread's entries are visible before its
-    // countdowns; the record that brings a count to zero completed its group.
-    uint32_t last = 0u;  // bit m: slot m's record completed its voxel's group
-    if (placed) {
-        __threadfence();
+    int total = 0;
 #pragma unroll
-        for (int m = 0; m < kGroupPerThread; ++m)
-            if (((placed >> m) & 1u) && atomicSub(&u.vcnt[vi[m]], 1u) == 1u) last |= 1u << m;
+    for (int m = 0; m < kGroupPerThread; ++m) {
+        const bool has = (cross >> m) & 1u;
+        const unsigned who = __ballot_sync(0xffffffffu, has);
+        if (has) queue[total + __popc(who & lanemask_lt())] = make_uint2(first + m, vi[m]);
+        total += __popc(who);
     }
-    // Every group completed here is selected by the whole warp, one at a
-    // time, lowest lane first.
-    while (__any_sync(0xffffffffu, last != 0u)) {
-        const int src = __ffs(__ballot_sync(0xffffffffu, last != 0u)) - 1;
-        uint32_t pick = kNoVoxel;
-        bool got = false;
-#pragma unroll
-        for (int m = 0; m < kGroupPerThread; ++m)
-            if (!got && ((last >> m) & 1u)) {
-                pick = vi[m];
-                got = true;
-            }
-        if (lane == src) last &= last - 1u;  // its lowest pending group
-        const uint32_t gv = __shfl_sync(0xffffffffu, pick, src);
-        if constexpr (S == kStoreF64)
-            updated += select_group<S>(select_args(v, u), v, a, gv, hist, lane);
-        else
-            updated += select_group_out<S>(select_args(v, u), gv, hist, lane);
-    }
+    __syncwarp();
+    for (int q = lane; q < total; q += 32) place_record<S>(v, a, u, queue[q].x, queue[q].y);
+    __syncwarp();  // the queue is rewritten by the warp's next slots
 }
 
 template <int S>
@@ -693,38 +645,13 @@ group_kernel(DevVolume v, BatchArgs a, UpdateScratch u, uint32_t n_slots) {
     launch_dependents();
     grid_dependency_wait();
     if (u.ctl->n_crossing == 0ull) return;  // no voxel crossed the cap in this batch
-    if (OSN_SPLIT_SELECT) {
-        // Placing only: no voxel is finished here, so there is nothing to
-        // count and no CTA barrier (each warp leaves when its slots are done).
-        if (OSN_GROUP_PERSISTENT) {
-            // Persistent grid: each thread walks chunks of eight slots a grid
-            // apart, the next chunk's records loaded before this one's are placed.
-            const uint32_t stride = gridDim.x * kGroupThreads * kGroupPerThread;
-            uint32_t first = (blockIdx.x * kGroupThreads + threadIdx.x) * kGroupPerThread;
-            uint32_t cur[kGroupPerThread], nxt[kGroupPerThread];
-            load_records(u, first, n_slots, cur);
-            for (; first < n_slots; first += stride) {
-                load_records(u, first + stride, n_slots, nxt);
-                place_records<S>(a, v, u, first, cur);
-#pragma unroll
-                for (int m = 0; m < kGroupPerThread; ++m) cur[m] = nxt[m];
-            }
-        } else {
-            const uint32_t first = (blockIdx.x * kGroupThreads + threadIdx.x) * kGroupPerThread;
-            uint32_t vi[kGroupPerThread];
-            load_records(u, first, n_slots, vi);
-            place_records<S>(a, v, u, first, vi);
-        }
-        return;
-    }
-    __shared__ uint32_t hist[kGroupWarps][256];
-    __shared__ int s_updated;
-    if (threadIdx.x == 0) s_updated = 0;
-    __syncthreads();
-    int updated = 0;
-    group_slots<S>(v, a, u, (blockIdx.x * kGroupThreads + threadIdx.x) * kGroupPerThread, n_slots,
-                   hist[threadIdx.x >> 5], updated);
-    cta_add(&s_updated, updated, &u.ctl->n_updated);
+    // Placing only: no voxel is finished here, so there is nothing to count
+    // and no CTA barrier (each warp leaves when its slots are done).
+    __shared__ uint2 queue[kGroupWarps][32 * kGroupPerThread];
+    const uint32_t first = (blockIdx.x * kGroupThreads + threadIdx.x) * kGroupPerThread;
+    uint32_t vi[kGroupPerThread];
+    load_records(u, first, n_slots, vi);
+    place_records<S>(a, v, u, first, vi, queue[threadIdx.x >> 5]);
 }
 
 constexpr int kSelectChunk = 32;   // voxels whose headers a warp loads together (one per lane)
@@ -836,7 +763,7 @@ __device__ __forceinline__ int select_stream(const SelectArgs& sa, const uint32_
 }
 
 // The ordered selection of every cap-crossing voxel of the batch, from the
-// list finish wrote (OSN_SPLIT_SELECT): warp w takes voxels w, w + warps,
+// list finish wrote: warp w takes voxels w, w + warps,
 // ... (so large groups spread over the grid); the FP64 oracle storage, one
 // voxel at a time.
 template <int S>
@@ -998,43 +925,36 @@ template <int S>
 __global__ void __launch_bounds__(kGroupThreads, OSN_GROUP_MIN_BLOCKS)
 group_multi_kernel(StepWork w) {
     __shared__ SceneWork sw;
-    __shared__ uint32_t hist[kGroupWarps][256];
+    __shared__ uint2 queue[kGroupWarps][32 * kGroupPerThread];
     __shared__ int s_begin[kMaxBatchScenes + 1];
-    __shared__ int s_item, s_updated;
-    const int t = threadIdx.x, lane = t & 31;
+    __shared__ int s_item;
+    const int t = threadIdx.x;
     launch_dependents();
     grid_dependency_wait();
-    if (t == 0) s_updated = 0;
     scene_prefix<kPassGroup>(w, s_begin);
     const int total = s_begin[w.n_scenes];
-    int cur = -1, updated = 0;
+    int cur = -1;
     for (;;) {
         if (t == 0) s_item = (int)atomicAdd(&w.queues[kQGroup], 1u);
         __syncthreads();
         const int item = s_item;
-        const bool done = item >= total;
-        const int sc = done ? -1 : scene_of(s_begin, w.n_scenes, item);
-        if (sc != cur || done) {
-            const int wsum = __reduce_add_sync(0xffffffffu, updated);
-            if (lane == 0 && wsum) atomicAdd(&s_updated, wsum);
-            __syncthreads();
-            if (t == 0 && cur >= 0 && s_updated) atomicAdd(&sw.u.ctl->n_updated, s_updated);
-            __syncthreads();
-            if (t == 0) s_updated = 0;
-            updated = 0;
-            if (done) break;
+        if (item >= total) break;  // also on a CTA's first pull when items are few
+        const int sc = scene_of(s_begin, w.n_scenes, item);
+        if (sc != cur) {
             cta_copy(&sw, &w.scenes[sc]);
             __syncthreads();
             cur = sc;
         }
         const uint32_t first = ((uint32_t)(item - s_begin[sc]) * kGroupThreads + t) * kGroupPerThread;
-        group_slots<S>(sw.v, sw.a, sw.u, first, (uint32_t)sw.n_slots, hist[t >> 5], updated);
-        __syncthreads();
+        uint32_t vi[kGroupPerThread];
+        load_records(sw.u, first, (uint32_t)sw.n_slots, vi);
+        place_records<S>(sw.a, sw.v, sw.u, first, vi, queue[t >> 5]);
+        __syncthreads();  // s_item and the descriptor are rewritten next
     }
 }
 
 // The ordered selection of every scene's cap-crossing voxels: warp work
-// items, one per listed voxel (OSN_SPLIT_SELECT).
+// items, one per listed voxel.
 template <int S>
 __global__ void __launch_bounds__(kSelectThreads)
 select_multi_kernel(StepWork w) {
@@ -1104,13 +1024,7 @@ cudaError_t launch_group(const DevVolume& v, const BatchArgs& a, const UpdateScr
     const uint32_t n_slots = (uint32_t)a.n * (2u * (uint32_t)v.steps + 1u);
     if (n_slots == 0) return cudaSuccess;
     const uint32_t per_cta = kGroupThreads * (uint32_t)kGroupPerThread;
-    uint32_t grid = (n_slots + per_cta - 1u) / per_cta;
-    if (OSN_SPLIT_SELECT && OSN_GROUP_PERSISTENT) {  // persistent: at most one resident wave
-        const int res = v.storage == kStoreF16U16 ? resident_grid<group_kernel<kStoreF16U16>>(kGroupThreads, sm_count)
-                        : v.storage == kStoreF64  ? resident_grid<group_kernel<kStoreF64>>(kGroupThreads, sm_count)
-                                                  : resident_grid<group_kernel<kStoreF32>>(kGroupThreads, sm_count);
-        grid = std::min<uint32_t>(grid, (uint32_t)res);
-    }
+    const uint32_t grid = (n_slots + per_cta - 1u) / per_cta;
     switch (v.storage) {
         case kStoreF16U16: return launch_after(group_kernel<kStoreF16U16>, grid, kGroupThreads, s, v, a, u, n_slots);
         case kStoreF64: return launch_after(group_kernel<kStoreF64>, grid, kGroupThreads, s, v, a, u, n_slots);
@@ -1120,7 +1034,6 @@ cudaError_t launch_group(const DevVolume& v, const BatchArgs& a, const UpdateScr
 
 cudaError_t launch_select(const DevVolume& v, const BatchArgs& a, const UpdateScratch& u, int sm_count,
                           cudaStream_t s) {
-    if (!OSN_SPLIT_SELECT) return cudaSuccess;  // the group pass selects
     switch (v.storage) {
         case kStoreF16U16:
             return launch_after(select_kernel<kStoreF16U16>,
@@ -1184,7 +1097,6 @@ cudaError_t launch_group_multi(const StepWork& w, int storage, int sm_count, cud
 
 namespace osn_b200 {
 cudaError_t launch_select_multi(const StepWork& w, int storage, int sm_count, cudaStream_t s) {
-    if (!OSN_SPLIT_SELECT) return cudaSuccess;  // the group pass selects
     switch (storage) {
         case kStoreF16U16: return select_multi_t<kStoreF16U16>(w, sm_count, s);
         case kStoreF64: return select_multi_t<kStoreF64>(w, sm_count, s);
