@@ -5,33 +5,49 @@
 // thread per cube, a full hash probe for each of the 8 corners of every cube
 // and one global atomic per emitting tetrahedron).
 //
-// B200 design. One CTA per block, one thread per cube, but the 7 neighbour
-// blocks are looked up once per CTA and the 9x9x9 halo of corner samples
-// (mean TSDF, validity, mean colour) is staged in shared memory with
-// coalesced reads, so the corner loop reads shared memory only. Emission is
-// compacted: each thread counts its vertices, a block-wide scan (warp
-// shuffles) gives every thread its offset, and one atomic per CTA reserves
-// the block's output range, so a block's triangles are contiguous and in a
-// fixed order (cube, then tetrahedron).
+// B200 design. A resident grid of 128-thread CTAs takes one block after the
+// other (the block count is read on the device). The 7 neighbour blocks are
+// looked up once per block and the 9x9x9 halo of corner samples (mean TSDF,
+// mean colour) is staged in shared memory, three rows of nine a warp, so that
+// two ballots give the rows' validity and below-iso bits. One warp finds the
+// cubes with a sign change from those bits, a row of eight cubes at a time
+// (about 45 of a block's 512), counts their triangles, reserves the block's
+// output range with one atomic and lists the triangles in a fixed order
+// (cube, then tetrahedron). Each warp then takes 32 triangles at a time, stages
+// their vertices and writes them out by itself.
+//
+// What bounds it: the latency of its instructions (36 M warp instructions for
+// 6,243 blocks and 1.34 M triangles, issue slots 47 % used at the 40 warps an SM
+// that the registers allow). A 512-thread CTA per block with a thread per cube
+// took 57 M and 120 us on a room of 8,468 blocks and 5.35 M vertices, against
+// 90; a quarter of its instructions listed triangles cube by cube, another
+// looked up the cases and ordered the corners of every edge. Looking the next
+// block up ahead of time changed nothing (90.5).
 //
 // Arithmetic follows the reference operation for operation, unfused, so a
 // volume whose voxels match bit-for-bit extracts bit-identical vertices.
 #include <algorithm>
+#include <mutex>
 
 #include "volume.h"
 
 namespace osn_b200 {
 namespace {
 
-constexpr int kExtractThreads = 512;
+constexpr int kExtractThreads = 128;
+constexpr int kExtractWarps = kExtractThreads / 32;
 constexpr int kResetThreads = 128;
 constexpr int kHalo = 9;
-constexpr int kHaloCells = kHalo * kHalo * kHalo;
+constexpr int kHaloRows = kHalo * kHalo;  // rows of nine cells along x
+constexpr int kHaloCells = kHaloRows * kHalo;
 
 // marching_tets.cpp:37-40: six tetrahedra around the 0-7 diagonal.
-constexpr int kTetCorners[6][4] = {
-    {0, 5, 1, 7}, {0, 1, 3, 7}, {0, 3, 2, 7}, {0, 6, 4, 7}, {0, 4, 5, 7}, {0, 2, 6, 7},
-};
+__host__ __device__ constexpr int tet_corner(int k, int i) {
+    constexpr int corners[6][4] = {
+        {0, 5, 1, 7}, {0, 1, 3, 7}, {0, 3, 2, 7}, {0, 6, 4, 7}, {0, 4, 5, 7}, {0, 2, 6, 7},
+    };
+    return corners[k][i];
+}
 
 // A tetrahedron's case code (bit i: its corner i is below iso) gives its
 // crossing (marching_tets.cpp:165-182): none (0000, 1111), one triangle from
@@ -41,23 +57,32 @@ constexpr int popc4(int x) { return (x & 1) + ((x >> 1) & 1) + ((x >> 2) & 1) + 
 constexpr int tris_of_code(int code) { return (popc4(code) & 1) ? 1 : (popc4(code) == 2 ? 2 : 0); }
 constexpr int tet_code(int below, int k) {
     int code = 0;
-    for (int i = 0; i < 4; ++i) code |= ((below >> kTetCorners[k][i]) & 1) << i;
+    for (int i = 0; i < 4; ++i) code |= ((below >> tet_corner(k, i)) & 1) << i;
     return code;
 }
 
+constexpr int corner_offset(int c) { return (c & 1) + ((c >> 1) & 1) * kHalo + ((c >> 2) & 1) * kHaloRows; }
+// The corner with the smaller position (x, then y, then z) comes first in an
+// interpolation (marching_tets.cpp:59-80). Corner positions are increasing
+// functions of the corner's offset bits on each axis (same cube), so comparing
+// the offsets (x, y, z) as a 3-bit number orders the positions exactly.
+constexpr int corner_rank(int c) { return ((c & 1) << 2) | (c & 2) | ((c >> 2) & 1); }
+
 // Tables the kernel stages in shared memory (constant-bank reads with lane-
 // dependent indices would serialise):
-//   kinds[below]   the six tetrahedra's triangle counts (2 bits each) of a
-//                  cube whose corners below iso are the bits of `below`;
-//   cases[k][code] tetrahedron k's corners (a, b, c, d) in the order the
-//                  case table of marching_tets.cpp:165-182 names them (3 bits
-//                  each) and its triangle count (bits 12-13);
-//   corners[k]     tetrahedron k's four corners (3 bits each).
-struct alignas(4) TetTables {
+//   kinds[below]     the six tetrahedra's triangle counts (2 bits each) of a
+//                    cube whose corners below iso are the bits of `below`;
+//   first[k][code]   the first of tetrahedron k's triangles in `tri`;
+//   tri[n]           a triangle's three edges, each as its two corners in
+//                    interpolation order: .x, .y their offsets in the halo (one
+//                    byte each), .z their offset bits (3 each).
+constexpr int kTetTris = 20;  // 8 codes of one triangle, 6 of two
+struct alignas(16) TetTables {
+    uint4 tri[6 * kTetTris];
     uint16_t kinds[256];
-    uint16_t cases[6][16];
-    uint16_t corners[6];
+    uint8_t first[6][16];
 };
+static_assert(sizeof(TetTables) % 4 == 0, "copied by words");
 constexpr int case_perm(int code) {  // (a, b, c, d) as positions in the tetrahedron
     switch (code) {
         case 0x01: case 0x0E: case 0x03: return 0 | 1 << 2 | 2 << 4 | 3 << 6;
@@ -72,6 +97,18 @@ constexpr int case_perm(int code) {  // (a, b, c, d) as positions in the tetrahe
         default: return 0;
     }
 }
+constexpr uint4 make_tri(const int (&edges)[3][2]) {
+    uint32_t off[2] = {0u, 0u}, bits = 0u;
+    for (int e = 0; e < 3; ++e) {
+        const bool swap = corner_rank(edges[e][1]) < corner_rank(edges[e][0]);
+        for (int i = 0; i < 2; ++i) {
+            const int c = edges[e][swap ? 1 - i : i], n = 2 * e + i;
+            off[n / 4] |= (uint32_t)corner_offset(c) << (8 * (n % 4));
+            bits |= (uint32_t)c << (3 * n);
+        }
+    }
+    return uint4{off[0], off[1], bits, 0u};
+}
 constexpr TetTables make_tet_tables() {
     TetTables t{};
     for (int b = 0; b < 256; ++b) {
@@ -79,15 +116,24 @@ constexpr TetTables make_tet_tables() {
         for (int k = 0; k < 6; ++k) v |= tris_of_code(tet_code(b, k)) << (2 * k);
         t.kinds[b] = (uint16_t)v;
     }
+    int n = 0;
     for (int k = 0; k < 6; ++k) {
-        int c = 0;
-        for (int i = 0; i < 4; ++i) c |= kTetCorners[k][i] << (3 * i);
-        t.corners[k] = (uint16_t)c;
         for (int code = 0; code < 16; ++code) {
             const int p = case_perm(code);
-            int e = 0;
-            for (int i = 0; i < 4; ++i) e |= kTetCorners[k][(p >> (2 * i)) & 3] << (3 * i);
-            t.cases[k][code] = (uint16_t)(e | tris_of_code(code) << 12);
+            const int a = tet_corner(k, p & 3), b = tet_corner(k, (p >> 2) & 3), c = tet_corner(k, (p >> 4) & 3),
+                      d = tet_corner(k, (p >> 6) & 3);
+            t.first[k][code] = (uint8_t)n;
+            // marching_tets.cpp:142-163: a single triangle (a-b, a-c, a-d), or
+            // the quad's two (a-c, a-d, b-d) and (a-c, b-d, b-c).
+            if (tris_of_code(code) == 1) {
+                const int e[3][2] = {{a, b}, {a, c}, {a, d}};
+                t.tri[n++] = make_tri(e);
+            } else if (tris_of_code(code) == 2) {
+                const int e0[3][2] = {{a, c}, {a, d}, {b, d}};
+                const int e1[3][2] = {{a, c}, {b, d}, {b, c}};
+                t.tri[n++] = make_tri(e0);
+                t.tri[n++] = make_tri(e1);
+            }
         }
     }
     return t;
@@ -95,59 +141,61 @@ constexpr TetTables make_tet_tables() {
 __constant__ TetTables c_tet_tables = make_tet_tables();
 static_assert(make_tet_tables().kinds[0] == 0 && make_tet_tables().kinds[255] == 0, "no crossing");
 static_assert(make_tet_tables().kinds[1] == 0x555, "corner 0 alone: one triangle in every tetrahedron");
+static_assert(make_tet_tables().first[5][15] == 6 * kTetTris, "every triangle has its place");
 
 // The block's 9^3 corner samples; colours only when the caller wants them.
 template <bool COL>
 struct Halo {
     float val[kHaloCells];
     float col[COL ? 3 : 1][COL ? kHaloCells : 1];
-    unsigned char flag[kHaloCells];  // bit 0: valid sample; bit 1: valid and below iso
+    uint32_t row[kHaloRows];  // bit x: cell x is valid; bit 16 + x: valid and below iso
 };
+
+// The eight cubes of row (ly, lz): bit x set where every corner of cube x is
+// valid and some but not all of them lie below iso.
+template <bool COL>
+__device__ __forceinline__ unsigned crossing_cubes(const Halo<COL>& h, int row) {
+    const int r0 = (row >> 3) * kHalo + (row & 7);
+    const uint32_t a = h.row[r0], b = h.row[r0 + 1], c = h.row[r0 + kHalo], d = h.row[r0 + kHalo + 1];
+    const uint32_t all = a & b & c & d, any = a | b | c | d;
+    const uint32_t both = all & (all >> 1), some = any | (any >> 1);
+    return (both & (some >> 16) & ~(both >> 16)) & 0xFFu;
+}
+
+// The corners of a cube that lie below iso (bit c: corner c).
+template <bool COL>
+__device__ __forceinline__ unsigned below_iso(const Halo<COL>& h, int cube) {
+    const int r0 = (cube >> 6) * kHalo + ((cube >> 3) & 7), x = 16 + (cube & 7);
+    return ((h.row[r0] >> x) & 3u) | ((h.row[r0 + 1] >> x) & 3u) << 2 | ((h.row[r0 + kHalo] >> x) & 3u) << 4 |
+           ((h.row[r0 + kHalo + 1] >> x) & 3u) << 6;
+}
 
 struct Cube {
-    int vx, vy, vz;  // voxel coordinate of corner 0
-    int h0;          // halo index of corner 0
-    float vs;
+    float lo[3], hi[3];  // voxel centres of corner 0 and corner 7 (marching_tets.cpp:126-128)
+    int h0;              // halo index of corner 0
 };
-
-__device__ __forceinline__ int corner_halo(const Cube& q, int c) {
-    return q.h0 + ((c >> 2) & 1) * kHalo * kHalo + ((c >> 1) & 1) * kHalo + (c & 1);
-}
-
-// Voxel centre of a corner (marching_tets.cpp:126-128).
-__device__ __forceinline__ void corner_pos(const Cube& q, int c, float p[3]) {
-    p[0] = __fmul_rn(__fadd_rn((float)(q.vx + (c & 1)), 0.5f), q.vs);
-    p[1] = __fmul_rn(__fadd_rn((float)(q.vy + ((c >> 1) & 1)), 0.5f), q.vs);
-    p[2] = __fmul_rn(__fadd_rn((float)(q.vz + ((c >> 2) & 1)), 0.5f), q.vs);
-}
 
 struct Vert {
     float p[3];
     float c[3];
 };
 
-// marching_tets.cpp:59-80: position-ordered interpolation.
+// marching_tets.cpp:59-80: position-ordered interpolation between two corners,
+// given by their halo indices and offset bits (first corner: bits 0-2).
 template <bool COL>
-__device__ __forceinline__ Vert interp(const Halo<COL>& h, const Cube& q, float iso, int ia, int ib) {
-    // The corner with the smaller position (x, then y, then z) first. Corner
-    // positions are increasing functions of the corner's offset bits on each
-    // axis (same cube), so comparing the offsets (x, y, z) as a 3-bit number
-    // orders the positions exactly.
-    const int ka = ((ia & 1) << 2) | (ia & 2) | ((ia >> 2) & 1);
-    const int kb = ((ib & 1) << 2) | (ib & 2) | ((ib >> 2) & 1);
-    const bool sw = kb < ka;
-    const int i0 = sw ? ib : ia, i1 = sw ? ia : ib;
-    float p0[3], p1[3];
-    corner_pos(q, i0, p0);
-    corner_pos(q, i1, p1);
-    const int h0 = corner_halo(q, i0), h1 = corner_halo(q, i1);
+__device__ __forceinline__ Vert interp(const Halo<COL>& h, const Cube& q, float iso, int h0, int h1, unsigned bits) {
     const float v0 = h.val[h0], v1 = h.val[h1];
     const float den = __fsub_rn(v1, v0);
     const float t = fabsf(den) < 1e-12f ? 0.5f : __fdiv_rn(__fsub_rn(iso, v0), den);
     const float tc = fminf(fmaxf(t, 0.0f), 1.0f);
     Vert o;
-    for (int k = 0; k < 3; ++k) o.p[k] = __fadd_rn(p0[k], __fmul_rn(tc, __fsub_rn(p1[k], p0[k])));
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const float p0 = (bits >> k) & 1u ? q.hi[k] : q.lo[k], p1 = (bits >> (3 + k)) & 1u ? q.hi[k] : q.lo[k];
+        o.p[k] = __fadd_rn(p0, __fmul_rn(tc, __fsub_rn(p1, p0)));
+    }
     if constexpr (COL) {
+#pragma unroll
         for (int k = 0; k < 3; ++k) {
             const float c0 = h.col[k][h0], c1 = h.col[k][h1];
             o.c[k] = __fadd_rn(c0, __fmul_rn(tc, __fsub_rn(c1, c0)));
@@ -156,36 +204,36 @@ __device__ __forceinline__ Vert interp(const Halo<COL>& h, const Cube& q, float 
     return o;
 }
 
-// Where a CTA's vertices go: the block's output range is contiguous, so its
-// first stage_verts vertices are staged in shared memory (with the range's
-// offset inside its 16-byte group, so the copy-out is aligned) and written
-// out by the whole CTA with 16-byte streaming stores; any further vertices
-// of an unusually dense block go straight to global memory. The instance
-// with colours stages fewer (its halo holds the colours too).
+// A warp's 32 triangles in shared memory, as they go to the output: 96
+// vertices of six floats (and 96 colours of three bytes), shifted by the
+// output's offset inside its 16-byte (4-byte) group so that the copy-out is
+// aligned on both sides.
+constexpr int kStageFloats = 32 * 18;
+constexpr int kStageBytes = 32 * 9;
 template <bool COL>
-__host__ __device__ constexpr int stage_verts() { return COL ? 1024 : 1536; }
-// A cube emits at most 6 tetrahedra x 2 triangles.
-constexpr int kMaxBlockTris = kBlockVoxels * 12;
-// Dynamic shared memory of one CTA: the vertex stage (pad + stage_verts * 6
-// floats), then the block's triangle list (one 16-bit item per triangle).
-template <bool COL>
-__host__ __device__ constexpr int extract_dyn_smem() {
-    return (4 + stage_verts<COL>() * 6) * 4 + kMaxBlockTris * 2;
-}
-template <bool COL>
-struct VertexSink {
-    float* stage;     // shared: [pad + stage_verts * 6]
-    int pad;          // floats of the 16-byte group before the block's first vertex
-    float* posnor;    // global output
-    int64_t base;     // the block's first vertex in the output
-    __device__ __forceinline__ float* slot(int local) const {
-        return local < stage_verts<COL>() ? stage + pad + local * 6 : posnor + (base + local) * 6;
-    }
+struct VertexStage {
+    alignas(16) float f[4 + kStageFloats];
+    alignas(4) uint8_t c[COL ? 4 + kStageBytes : 4];
 };
 
+// n elements of T staged at s[pad ...] to out, whose first element lies pad
+// elements into an aligned group of sizeof(V): whole groups as one V, the
+// partial first and last ones by element.
+template <typename V, typename T>
+__device__ __forceinline__ void copy_out(T* out, const T* s, int pad, int n, int lane) {
+    constexpr int kPer = (int)(sizeof(V) / sizeof(T));
+    const int head = min(n, (kPer - pad) & (kPer - 1));  // elements before the first whole group
+    const int groups = (n - head) / kPer, tail = n - head - groups * kPer;
+    const V* from = reinterpret_cast<const V*>(s + pad + head);
+    V* to = reinterpret_cast<V*>(out + head);
+#pragma unroll 5
+    for (int g = lane; g < groups; g += 32) __stcs(to + g, from[g]);
+    if (lane < head) out[lane] = s[pad + lane];
+    if (lane < tail) out[n - tail + lane] = s[pad + n - tail + lane];
+}
+
 template <bool COL>
-__device__ __forceinline__ void emit_triangle(const Vert& a, const Vert& b, const Vert& c,
-                                              const VertexSink<COL>& out, uint8_t* rgb, int local) {
+__device__ __forceinline__ void stage_triangle(const Vert& a, const Vert& b, const Vert& c, float* f, uint8_t* col) {
     // marching_tets.cpp:206-218: face normal of the emitted triangle.
     const float e1[3] = {__fsub_rn(b.p[0], a.p[0]), __fsub_rn(b.p[1], a.p[1]), __fsub_rn(b.p[2], a.p[2])};
     const float e2[3] = {__fsub_rn(c.p[0], a.p[0]), __fsub_rn(c.p[1], a.p[1]), __fsub_rn(c.p[2], a.p[2])};
@@ -200,8 +248,9 @@ __device__ __forceinline__ void emit_triangle(const Vert& a, const Vert& b, cons
         nz = __fdiv_rn(nz, len);
     }
     const Vert* vs[3] = {&a, &b, &c};
+#pragma unroll
     for (int k = 0; k < 3; ++k) {
-        float* dst = out.slot(local + k);
+        float* dst = f + 6 * k;
         dst[0] = vs[k]->p[0];
         dst[1] = vs[k]->p[1];
         dst[2] = vs[k]->p[2];
@@ -209,206 +258,238 @@ __device__ __forceinline__ void emit_triangle(const Vert& a, const Vert& b, cons
         dst[4] = ny;
         dst[5] = nz;
         if constexpr (COL) {
-            uint8_t* cc = rgb + (out.base + local + k) * 3;
-            cc[0] = (uint8_t)fminf(fmaxf(vs[k]->c[0], 0.0f), 255.0f);
-            cc[1] = (uint8_t)fminf(fmaxf(vs[k]->c[1], 0.0f), 255.0f);
-            cc[2] = (uint8_t)fminf(fmaxf(vs[k]->c[2], 0.0f), 255.0f);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) col[3 * k + j] = (uint8_t)fminf(fmaxf(vs[k]->c[j], 0.0f), 255.0f);
         }
     }
 }
 
-// Resident CTAs per SM the colourless instance is sized for: 4 x 512 threads
-// at 32 registers (a few bytes spill), measured 0.38 ms against 0.56 ms at 3
-// CTAs and 0.62 ms at 2 on a 14k-block, 8.7M-vertex mesh.
+// Triangles listed at a time (a few hundred are usual; an unusually dense
+// block takes several passes): room for 32 cubes of 6 tetrahedra x 2.
+constexpr int kListItems = 1024;
+static_assert(kListItems >= 32 * 12, "32 cubes fit the list");
+
+__device__ __forceinline__ int tri_count(unsigned kinds) { return __popc(kinds & 0x555u) + 2 * __popc(kinds & 0xAAAu); }
+
+// List the triangles of cubes[from ...] in output order (cube, tetrahedron,
+// triangle), 32 cubes at a time while the list has room, by one warp. Returns
+// the first cube left; listed: the triangles listed. An item is cube |
+// triangle in the table << 9.
+template <bool COL>
+__device__ __forceinline__ int list_triangles(const Halo<COL>& h, const TetTables& tab, const uint16_t* cubes, int from,
+                                              int n_cubes, uint16_t* items, int& listed, int lane) {
+    int n = 0, c0 = from;
+    for (; c0 < n_cubes; c0 += 32) {
+        const int cube = c0 + lane < n_cubes ? cubes[c0 + lane] : -1;
+        const unsigned bl = cube >= 0 ? below_iso(h, cube) : 0u;
+        const unsigned kinds = tab.kinds[bl];
+        const int tris = tri_count(kinds);
+        int upto = tris;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += y;
+        }
+        const int here = __shfl_sync(0xffffffffu, upto, 31);
+        if (n + here > kListItems) break;  // warp-uniform
+        int pos = n + upto - tris;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            const unsigned kind = (kinds >> (2 * k)) & 3u;
+            if (kind == 0u) continue;
+            const unsigned code = ((bl >> tet_corner(k, 0)) & 1u) | ((bl >> tet_corner(k, 1)) & 1u) << 1 |
+                                  ((bl >> tet_corner(k, 2)) & 1u) << 2 | ((bl >> tet_corner(k, 3)) & 1u) << 3;
+            const unsigned item = (unsigned)cube | (unsigned)tab.first[k][code] << 9;
+            items[pos++] = (uint16_t)item;
+            if (kind == 2u) items[pos++] = (uint16_t)(item + (1u << 9));
+        }
+        n += here;
+    }
+    listed = n;
+    return min(c0, n_cubes);
+}
+
+// Resident CTAs per SM the registers are sized for: 10 (48 registers; 90 us on
+// the room mesh, 99 at 11 and 100 at 12, which spill); with colours 7.
 #ifndef OSN_EXTRACT_MIN_BLOCKS
-#define OSN_EXTRACT_MIN_BLOCKS 4
+#define OSN_EXTRACT_MIN_BLOCKS 10
 #endif
+#ifndef OSN_EXTRACT_COL_MIN_BLOCKS
+#define OSN_EXTRACT_COL_MIN_BLOCKS 7
+#endif
+// Blocks: pool indices 0 .. *count - 1, or the *count entries of a list.
 template <int S, bool COL>
-__global__ void __launch_bounds__(kExtractThreads, COL ? 1 : OSN_EXTRACT_MIN_BLOCKS)
-extract_kernel(DevVolume v, int32_t n_blocks, const int32_t* list, float min_w, float iso, float* out_posnor,
+__global__ void __launch_bounds__(kExtractThreads, COL ? OSN_EXTRACT_COL_MIN_BLOCKS : OSN_EXTRACT_MIN_BLOCKS)
+extract_kernel(DevVolume v, const int32_t* list, const int32_t* count, float min_w, float iso, float* out_posnor,
                uint8_t* out_rgb, int32_t cap, int32_t* ctl) {
     __shared__ Halo<COL> h;
-    __shared__ uint8_t s_below[kBlockVoxels];
     __shared__ TetTables s_tab;
-    extern __shared__ __align__(16) float s_dyn[];
-    float* const s_stage = s_dyn;
-    uint16_t* const s_items = reinterpret_cast<uint16_t*>(s_dyn + 4 + stage_verts<COL>() * 6);
+    __shared__ uint16_t s_items[kListItems];
+    __shared__ uint16_t s_cubes[kBlockVoxels];  // the block's cubes with a sign change, ascending
+    __shared__ VertexStage<COL> s_stage[kExtractWarps];
+    __shared__ uint16_t s_cell[kHaloRows];  // first voxel of a halo row in its block | neighbour << 9
     __shared__ int s_nb[8];
-    __shared__ int s_warp[kExtractThreads / 32];
-    __shared__ int s_base, s_total;
+    __shared__ int s_base, s_tris, s_next;
+    __shared__ int s_cube_count, s_listed, s_upto;  // cubes, triangles listed, cubes they cover
 
-    if ((int)blockIdx.x >= n_blocks) return;
-    const int b = list ? list[blockIdx.x] : (int)blockIdx.x;  // the block's pool index
-    const int t = threadIdx.x;
-    const BlockCoord bc = v.block_coord[b];
-    if (t < 8) {
-        const int dx = t & 1, dy = (t >> 1) & 1, dz = (t >> 2) & 1;
-        const int nx = bc.x + dx, ny = bc.y + dy, nz = bc.z + dz;
-        s_nb[t] = t == 0 ? b : find_block(v, nx, ny, nz, pack_key(nx, ny, nz));
-    }
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     for (int k = t; k < (int)(sizeof(TetTables) / 4); k += kExtractThreads)
         reinterpret_cast<uint32_t*>(&s_tab)[k] = reinterpret_cast<const uint32_t*>(&c_tet_tables)[k];
-    __syncthreads();
+    if (t < kHaloRows) {
+        const int hy = t % kHalo, hz = t / kHalo;
+        s_cell[t] = (uint16_t)(((hz & 7) * kBlockDim + (hy & 7)) * kBlockDim | (hy >> 3) << 10 | (hz >> 3) << 11);
+    }
+    const int32_t n_blocks = min(*count, v.pool_capacity);
+    const int row3 = lane / kHalo, hx = lane - row3 * kHalo;  // this lane's place among three halo rows
+    // The warp that lists: not the same one in every CTA, whose warps of one
+    // number share a scheduler.
+    const int lister = blockIdx.x % kExtractWarps;
 
-    // Stage the halo: corner samples of this block plus the +x/+y/+z faces,
-    // edges and corner of its neighbours (volume.cpp:306-329 per sample).
-    for (int k = t; k < kHaloCells; k += kExtractThreads) {
-        const int hx = k % kHalo, hy = (k / kHalo) % kHalo, hz = k / (kHalo * kHalo);
-        const int nb = s_nb[(hx >> 3) | ((hy >> 3) << 1) | ((hz >> 3) << 2)];
-        unsigned char flag = 0;
-        h.val[k] = 0.0f;
-        if (nb >= 0) {
-            const size_t idx = (size_t)nb * kBlockVoxels + (size_t)((((hz & 7) * kBlockDim) + (hy & 7)) * kBlockDim + (hx & 7));
-            // Weight and stored TSDF loaded together (one round trip).
-            const float w = weight_at<S>(v, idx);
-            const float m = mean_from<S>(v, idx, w);
-            if (!(w < min_w || w <= 0.0f)) {
-                flag = m < iso ? 3 : 1;
-                h.val[k] = m;
-                if constexpr (COL) {
-                    if constexpr (S == kStoreF32) {
-                        const float inv = __fdiv_rn(1.0f, w);
-                        h.col[0][k] = __fmul_rn(v.r[idx], inv);
-                        h.col[1][k] = __fmul_rn(v.g[idx], inv);
-                        h.col[2][k] = __fmul_rn(v.b[idx], inv);
-                    } else {
-                        // No colour arrays: every contribution is grey.
-                        h.col[0][k] = 128.0f;
-                        h.col[1][k] = 128.0f;
-                        h.col[2][k] = 128.0f;
+    for (int32_t at = blockIdx.x; at < n_blocks;) {
+        const int b = list ? list[at] : at;  // the block's pool index
+        const BlockCoord bc = v.block_coord[b];
+        int next = 0;
+        if (t < 8) {
+            const int nx = bc.x + (t & 1), ny = bc.y + ((t >> 1) & 1), nz = bc.z + ((t >> 2) & 1);
+            s_nb[t] = t == 0 ? b : find_block(v, nx, ny, nz, pack_key(nx, ny, nz));
+        } else if (t == 32) {
+            next = (int)gridDim.x + atomicAdd(&ctl[2], 1);  // blocks differ in work: dealt out one by one
+        }
+        __syncthreads();  // also: every warp is done with the previous block
+
+        // Stage the halo: corner samples of this block plus the +x/+y/+z faces,
+        // edges and corner of its neighbours (volume.cpp:306-329 per sample).
+#pragma unroll
+        for (int i = 0; i < (kHaloRows / 3 + kExtractWarps - 1) / kExtractWarps; ++i) {
+            const int r = 3 * (warp + i * kExtractWarps);
+            if (r >= kHaloRows) break;  // warp-uniform
+            const int row = r + row3;
+            bool valid = false, below = false;
+            if (row3 < 3) {
+                const int cell = s_cell[row];
+                const int nb = s_nb[(cell >> 9) | (hx >> 3)];
+                float val = 0.0f;
+                if (nb >= 0) {
+                    const size_t idx = (size_t)nb * kBlockVoxels + (size_t)((cell & 511) | (hx & 7));
+                    // Weight and stored TSDF loaded together (one round trip).
+                    const float w = weight_at<S>(v, idx);
+                    const float m = mean_from<S>(v, idx, w);
+                    valid = !(w < min_w || w <= 0.0f);
+                    below = valid && m < iso;
+                    if (valid) {
+                        val = m;
+                        if constexpr (COL) {
+                            const int k = row * kHalo + hx;
+                            if constexpr (S == kStoreF32) {
+                                const float inv = __fdiv_rn(1.0f, w);
+                                h.col[0][k] = __fmul_rn(v.r[idx], inv);
+                                h.col[1][k] = __fmul_rn(v.g[idx], inv);
+                                h.col[2][k] = __fmul_rn(v.b[idx], inv);
+                            } else {
+                                // No colour arrays: every contribution is grey.
+                                h.col[0][k] = 128.0f;
+                                h.col[1][k] = 128.0f;
+                                h.col[2][k] = 128.0f;
+                            }
+                        }
                     }
                 }
+                h.val[row * kHalo + hx] = val;
             }
+            const unsigned vb = __ballot_sync(0xffffffffu, valid), bb = __ballot_sync(0xffffffffu, below);
+            if (lane < 3)
+                h.row[r + lane] = ((vb >> (kHalo * lane)) & 0x1FFu) | ((bb >> (kHalo * lane)) & 0x1FFu) << 16;
         }
-        h.flag[k] = flag;
-    }
-    __syncthreads();
+        if (t == 32) s_next = next;
+        __syncthreads();
 
-    Cube q;
-    const int lx = t & 7, ly = (t >> 3) & 7, lz = t >> 6;
-    q.vx = bc.x * kBlockDim + lx;
-    q.vy = bc.y * kBlockDim + ly;
-    q.vz = bc.z * kBlockDim + lz;
-    q.h0 = (lz * kHalo + ly) * kHalo + lx;
-    q.vs = v.voxel_size;
-
-    unsigned all_ok = 1u;
-    unsigned below = 0;  // bit c set when corner c is below iso
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-        const unsigned f = h.flag[corner_halo(q, c)];
-        all_ok &= f;
-        below |= (f >> 1) << c;
-    }
-
-    // Triangles of this cube (every corner valid, or none).
-    const unsigned kinds = (all_ok & 1u) ? s_tab.kinds[below] : 0u;
-    const int n_tri = __popc(kinds & 0x555u) + 2 * __popc(kinds & 0xAAAu);
-    s_below[t] = (uint8_t)below;
-
-    // Block-wide exclusive scan of the triangle counts.
-    const int lane = t & 31, warp = t >> 5;
-    int x = n_tri;
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) s_warp[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        int w = lane < kExtractThreads / 32 ? s_warp[lane] : 0;
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= o) w += y;
-        }
-        if (lane < kExtractThreads / 32) s_warp[lane] = w;
-        if (lane == kExtractThreads / 32 - 1) {
-            const int total = 3 * w;  // vertices
+        // The list, by one warp: cubes with a sign change in ascending order
+        // (two rows of cubes per lane), then their triangles.
+        if (warp == lister) {
+            const unsigned m0 = crossing_cubes(h, 2 * lane), m1 = crossing_cubes(h, 2 * lane + 1);
+            unsigned cubes = m0 | m1 << 8;
+            int incl = __popc(cubes);
+            const int own = incl;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += y;
+            }
+            const int n_cubes = __shfl_sync(0xffffffffu, incl, 31);
+            for (int pos = incl - own; cubes != 0u; cubes &= cubes - 1u, ++pos)
+                s_cubes[pos] = (uint16_t)(16 * lane + __ffs(cubes) - 1);
+            __syncwarp();
+            int n_tris = 0;
+            for (int c0 = 0; c0 < n_cubes; c0 += 32) {
+                const unsigned kinds = c0 + lane < n_cubes ? s_tab.kinds[below_iso(h, s_cubes[c0 + lane])] : 0u;
+                n_tris += __reduce_add_sync(0xffffffffu, tri_count(kinds));
+            }
             int base = 0;
-            if (total > 0) {
-                base = atomicAdd(&ctl[0], total);
-                if ((int64_t)base + total > (int64_t)cap) {
+            if (lane == 0 && n_tris > 0) base = atomicAdd(&ctl[0], 3 * n_tris);
+            int listed;
+            const int upto = list_triangles(h, s_tab, s_cubes, 0, n_cubes, s_items, listed, lane);
+            if (lane == 0) {
+                if ((int64_t)base + 3 * n_tris > (int64_t)cap) {
                     atomicExch(&ctl[1], 1);
                     base = -1;
                 }
+                s_base = base;
+                s_tris = n_tris;
+                s_cube_count = n_cubes;
+                s_listed = listed;
+                s_upto = upto;
             }
-            s_base = base;
-            s_total = total;
         }
-    }
-    __syncthreads();
-    const int total = s_total;
-    if (s_base < 0 || total == 0) return;  // uniform across the CTA
-    VertexSink<COL> sink;
-    sink.stage = s_stage;
-    // The caller's buffer is float-aligned, not necessarily 16-byte aligned:
-    // the pad is taken from the address of the block's first float.
-    sink.pad = (int)((reinterpret_cast<uintptr_t>(out_posnor + (int64_t)s_base * 6) >> 2) & 3);
-    sink.posnor = out_posnor;
-    sink.base = s_base;
+        __syncthreads();
+        at = s_next;
+        const int base = s_base;
+        if (s_tris == 0 || base < 0) continue;  // uniform: nothing here, or the block's vertices do not fit
 
-    // The block's triangle list in output order (cube, tetrahedron, triangle):
-    // item = cube | tetrahedron << 9 | second triangle of a quad << 12.
-    {
-        int at = (warp ? s_warp[warp - 1] : 0) + x - n_tri;
-        for (int k = 0; k < (n_tri > 0 ? 6 : 0); ++k) {
-            const int kind = (int)(kinds >> (2 * k)) & 3;
-            for (int m = 0; m < kind; ++m) s_items[at++] = (uint16_t)(t | k << 9 | m << 12);
-        }
-    }
-    __syncthreads();
-
-    // One thread per triangle: the warps stay converged however sparse the
-    // surface is within the block.
-    const int n_tris = total / 3;
-    for (int j = t; j < n_tris; j += kExtractThreads) {
-        const int item = s_items[j];
-        const int cube = item & (kBlockVoxels - 1), k = (item >> 9) & 7, second = item >> 12;
-        Cube qc;
-        const int cx = cube & 7, cy = (cube >> 3) & 7, cz = cube >> 6;
-        qc.vx = bc.x * kBlockDim + cx;
-        qc.vy = bc.y * kBlockDim + cy;
-        qc.vz = bc.z * kBlockDim + cz;
-        qc.h0 = (cz * kHalo + cy) * kHalo + cx;
-        qc.vs = v.voxel_size;
-        const unsigned bl = s_below[cube];
-        const unsigned tc = s_tab.corners[k];
-        const int code = (int)(((bl >> (tc & 7u)) & 1u) | (((bl >> ((tc >> 3) & 7u)) & 1u) << 1) |
-                               (((bl >> ((tc >> 6) & 7u)) & 1u) << 2) | (((bl >> (tc >> 9)) & 1u) << 3));
-        const unsigned e = s_tab.cases[k][code];
-        const int a = (int)(e & 7u), bb = (int)((e >> 3) & 7u), c = (int)((e >> 6) & 7u), d = (int)((e >> 9) & 7u);
-        // marching_tets.cpp:142-163: a single triangle (a-b, a-c, a-d), or the
-        // quad's two (a-c, a-d, b-d) and (a-c, b-d, b-c).
-        int e0a = a, e0b = c, e1a = a, e1b = d, e2a = bb, e2b = d;
-        if ((e >> 12) == 1u) {
-            e0b = bb;
-            e1b = c;
-            e2a = a;
-        } else if (second) {
-            e1a = bb;
-            e2b = c;
-        }
-        const Vert v0 = interp(h, qc, iso, e0a, e0b);
-        const Vert v1 = interp(h, qc, iso, e1a, e1b);
-        const Vert v2 = interp(h, qc, iso, e2a, e2b);
-        emit_triangle<COL>(v0, v1, v2, sink, out_rgb, 3 * j);
-    }
-    __syncthreads();
-    // Copy-out of the staged vertices: 16-byte groups of the output, each
-    // wholly inside the block's range stored as one vector, the partial
-    // first and last groups float by float.
-    const int n_floats = min(total, stage_verts<COL>()) * 6;
-    // The 16-byte group holding the block's first float; only floats of the
-    // block's range [pad, pad + n_floats) are written.
-    float* gbase = reinterpret_cast<float*>(reinterpret_cast<uintptr_t>(out_posnor + (int64_t)s_base * 6) -
-                                            4 * (uintptr_t)sink.pad);
-    const int groups = (sink.pad + n_floats + 3) >> 2;
-    for (int g = t; g < groups; g += kExtractThreads) {
-        const int lo = 4 * g;
-        if (lo >= sink.pad && lo + 4 <= sink.pad + n_floats) {
-            __stcs(reinterpret_cast<float4*>(gbase) + g, reinterpret_cast<const float4*>(s_stage)[g]);
-        } else {
-            for (int j = max(lo, sink.pad); j < min(lo + 4, sink.pad + n_floats); ++j) gbase[j] = s_stage[j];
+        for (int from = 0;;) {  // one pass, unless the block's list is longer than the stage
+            const int listed = s_listed, cubes_done = s_upto;
+            // One thread per triangle, 32 consecutive ones per warp.
+            VertexStage<COL>& stage = s_stage[warp];
+            for (int j0 = 32 * warp; j0 < listed; j0 += kExtractThreads) {
+                float* const out = out_posnor + ((int64_t)base + 3 * (from + j0)) * 6;
+                uint8_t* const out_c = COL ? out_rgb + ((int64_t)base + 3 * (from + j0)) * 3 : nullptr;
+                // The caller's buffers are aligned to their elements only.
+                const int pad = (int)((reinterpret_cast<uintptr_t>(out) >> 2) & 3);
+                const int pad_c = (int)(reinterpret_cast<uintptr_t>(out_c) & 3);
+                if (j0 + lane < listed) {
+                    const int item = s_items[j0 + lane];
+                    const int cube = item & (kBlockVoxels - 1);
+                    const uint4 tri = s_tab.tri[item >> 9];
+                    const int cc[3] = {cube & 7, (cube >> 3) & 7, cube >> 6};
+                    const int bo[3] = {bc.x, bc.y, bc.z};
+                    Cube q;
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) {
+                        const int vox = bo[a] * kBlockDim + cc[a];
+                        q.lo[a] = __fmul_rn(__fadd_rn((float)vox, 0.5f), v.voxel_size);
+                        q.hi[a] = __fmul_rn(__fadd_rn((float)(vox + 1), 0.5f), v.voxel_size);
+                    }
+                    q.h0 = (cc[2] * kHalo + cc[1]) * kHalo + cc[0];
+                    const Vert v0 = interp(h, q, iso, q.h0 + (int)(tri.x & 255u), q.h0 + (int)((tri.x >> 8) & 255u), tri.z);
+                    const Vert v1 = interp(h, q, iso, q.h0 + (int)((tri.x >> 16) & 255u), q.h0 + (int)(tri.x >> 24), tri.z >> 6);
+                    const Vert v2 = interp(h, q, iso, q.h0 + (int)(tri.y & 255u), q.h0 + (int)(tri.y >> 8), tri.z >> 12);
+                    stage_triangle<COL>(v0, v1, v2, stage.f + pad + 18 * lane, stage.c + pad_c + 9 * lane);
+                }
+                __syncwarp();
+                const int n = min(32, listed - j0);
+                copy_out<float4>(out, stage.f, pad, 18 * n, lane);
+                if constexpr (COL) copy_out<uint32_t>(out_c, stage.c, pad_c, 9 * n, lane);
+                __syncwarp();  // the stage is rewritten
+            }
+            if (cubes_done >= s_cube_count) break;  // uniform
+            __syncthreads();
+            from += listed;
+            if (warp == lister) {
+                int n;
+                const int upto = list_triangles(h, s_tab, s_cubes, cubes_done, s_cube_count, s_items, n, lane);
+                if (lane == 0) {
+                    s_listed = n;
+                    s_upto = upto;
+                }
+            }
+            __syncthreads();
         }
     }
 }
@@ -475,32 +556,36 @@ static_assert(kEmptyKey == -1, "an empty slot's key is all ones");
 }  // namespace
 
 template <int S, bool COL>
-static cudaError_t launch_extract_as(const DevVolume& v, int32_t n_blocks, const int32_t* list, float min_w,
-                                     float iso, float* posnor, uint8_t* rgb, int32_t cap, int32_t* ctl,
+static cudaError_t launch_extract_as(const DevVolume& v, const int32_t* list, const int32_t* count, float min_w,
+                                     float iso, float* posnor, uint8_t* rgb, int32_t cap, int32_t* ctl, int sm_count,
                                      cudaStream_t s) {
-    constexpr int dyn = extract_dyn_smem<COL>();
-    cudaError_t e = cudaFuncSetAttribute(extract_kernel<S, COL>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn);
-    if (e != cudaSuccess) return e;
-    extract_kernel<S, COL><<<n_blocks, kExtractThreads, dyn, s>>>(v, n_blocks, list, min_w, iso, posnor, rgb, cap, ctl);
+    static int per_sm = 0;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, extract_kernel<S, COL>, kExtractThreads, 0) !=
+                cudaSuccess ||
+            per_sm < 1)
+            per_sm = 1;
+    });
+    extract_kernel<S, COL><<<per_sm * sm_count, kExtractThreads, 0, s>>>(v, list, count, min_w, iso, posnor, rgb, cap, ctl);
     return cudaGetLastError();
 }
 
-cudaError_t launch_extract(const DevVolume& v, int32_t n_blocks, const int32_t* list, float min_w, float iso,
-                           float* posnor, uint8_t* rgb, int32_t cap, int32_t* ctl, cudaStream_t s) {
-    if (n_blocks <= 0) return cudaSuccess;
+cudaError_t launch_extract(const DevVolume& v, const int32_t* list, const int32_t* count, float min_w, float iso,
+                           float* posnor, uint8_t* rgb, int32_t cap, int32_t* ctl, int sm_count, cudaStream_t s) {
     // Colours in a separate instance: without them the halo holds a quarter
     // of the shared memory and the kernel fewer registers.
     const bool col = rgb != nullptr;
     switch (v.storage) {
         case kStoreF16U16:
-            return col ? launch_extract_as<kStoreF16U16, true>(v, n_blocks, list, min_w, iso, posnor, rgb, cap, ctl, s)
-                       : launch_extract_as<kStoreF16U16, false>(v, n_blocks, list, min_w, iso, posnor, nullptr, cap, ctl, s);
+            return col ? launch_extract_as<kStoreF16U16, true>(v, list, count, min_w, iso, posnor, rgb, cap, ctl, sm_count, s)
+                       : launch_extract_as<kStoreF16U16, false>(v, list, count, min_w, iso, posnor, nullptr, cap, ctl, sm_count, s);
         case kStoreF64:
-            return col ? launch_extract_as<kStoreF64, true>(v, n_blocks, list, min_w, iso, posnor, rgb, cap, ctl, s)
-                       : launch_extract_as<kStoreF64, false>(v, n_blocks, list, min_w, iso, posnor, nullptr, cap, ctl, s);
+            return col ? launch_extract_as<kStoreF64, true>(v, list, count, min_w, iso, posnor, rgb, cap, ctl, sm_count, s)
+                       : launch_extract_as<kStoreF64, false>(v, list, count, min_w, iso, posnor, nullptr, cap, ctl, sm_count, s);
         default:
-            return col ? launch_extract_as<kStoreF32, true>(v, n_blocks, list, min_w, iso, posnor, rgb, cap, ctl, s)
-                       : launch_extract_as<kStoreF32, false>(v, n_blocks, list, min_w, iso, posnor, nullptr, cap, ctl, s);
+            return col ? launch_extract_as<kStoreF32, true>(v, list, count, min_w, iso, posnor, rgb, cap, ctl, sm_count, s)
+                       : launch_extract_as<kStoreF32, false>(v, list, count, min_w, iso, posnor, nullptr, cap, ctl, sm_count, s);
     }
 }
 

@@ -103,7 +103,7 @@ bool Volume::alloc_device(uint32_t hash_slots) {
     OSN_TRY(cudaMalloc(&us_.touched, (size_t)dv_.pool_capacity * sizeof(int32_t)));
     OSN_TRY(cudaMalloc(&us_.ctl, sizeof(UpdateControl)));
     us_.status = dv_.status;
-    OSN_TRY(cudaMalloc(&mesh_ctl_, 2 * sizeof(int32_t)));
+    OSN_TRY(cudaMalloc(&mesh_ctl_, kMeshCounters * sizeof(int32_t)));
     if (dv_.slot_index) {
         OSN_TRY(cudaMalloc(&block_list_, (size_t)dv_.pool_capacity * sizeof(int32_t)));
         OSN_TRY(cudaMalloc(&list_count_, sizeof(int32_t)));
@@ -442,8 +442,6 @@ bool Volume::ensure_mesh(int32_t cap, bool rgb) {
 int32_t Volume::extract(float* posnor, uint8_t* rgb, int32_t cap, float min_w, float iso,
                         bool host_out) {
     join();
-    const int32_t n_blocks = block_count();  // waits for the stream
-    if (n_blocks <= 0) return 0;
     float* d_pos = posnor;
     uint8_t* d_rgb = rgb;
     if (host_out) {
@@ -451,12 +449,12 @@ int32_t Volume::extract(float* posnor, uint8_t* rgb, int32_t cap, float min_w, f
         d_pos = mesh_posnor_;
         d_rgb = rgb ? mesh_rgb_ : nullptr;
     }
-    if (cudaMemsetAsync(mesh_ctl_, 0, 2 * sizeof(int32_t), stream_) != cudaSuccess) return -1;
-    const int32_t nb = std::min(n_blocks, dv_.pool_capacity);
-    const int32_t* list = block_list(nb);
-    if (dv_.slot_index && !list) return -1;
+    if (cudaMemsetAsync(mesh_ctl_, 0, kMeshCounters * sizeof(int32_t), stream_) != cudaSuccess) return -1;
+    Blocks blocks;
+    if (allocated_blocks(blocks) != cudaSuccess) return -1;
     mark_start(kKExtract);
-    const cudaError_t e = launch_extract(dv_, nb, list, min_w, iso, d_pos, d_rgb, cap, mesh_ctl_, stream_);
+    const cudaError_t e = launch_extract(dv_, blocks.list, blocks.count, min_w, iso, d_pos, d_rgb, cap, mesh_ctl_,
+                                         sm_count_, stream_);
     mark_end(kKExtract);
     if (e != cudaSuccess) return -1;
     int32_t* hs = reinterpret_cast<int32_t*>(host_small_);
@@ -478,12 +476,12 @@ int32_t Volume::extract(float* posnor, uint8_t* rgb, int32_t cap, float min_w, f
     return n;
 }
 
-const int32_t* Volume::block_list(int32_t n) {
-    if (!dv_.slot_index || n <= 0) return nullptr;
-    if (cudaMemsetAsync(list_count_, 0, sizeof(int32_t), stream_) != cudaSuccess ||
-        launch_list_blocks(dv_, block_list_, list_count_, stream_) != cudaSuccess)
-        return nullptr;
-    return block_list_;
+cudaError_t Volume::allocated_blocks(Blocks& out) {
+    out = Blocks{nullptr, dv_.block_count};
+    if (!dv_.slot_index) return cudaSuccess;
+    out = Blocks{block_list_, list_count_};
+    const cudaError_t e = cudaMemsetAsync(list_count_, 0, sizeof(int32_t), stream_);
+    return e == cudaSuccess ? launch_list_blocks(dv_, block_list_, list_count_, stream_) : e;
 }
 
 bool Volume::reserve_batch(int32_t max_points) {
@@ -510,15 +508,10 @@ SceneWork Volume::batch_work(const BatchArgs& a, cudaStream_t s) {
 
 cudaError_t Volume::reset() {
     join();
-    cudaError_t e = cudaSuccess;
     mark_start(kKReset);
-    if (dv_.slot_index) {  // the occupied slots, before the table is cleared
-        e = cudaMemsetAsync(list_count_, 0, sizeof(int32_t), stream_);
-        if (e == cudaSuccess) e = launch_list_blocks(dv_, block_list_, list_count_, stream_);
-        if (e == cudaSuccess) e = launch_reset(dv_, block_list_, list_count_, stream_);
-    } else {
-        e = launch_reset(dv_, nullptr, dv_.block_count, stream_);
-    }
+    Blocks blocks;  // listed before the table is cleared
+    cudaError_t e = allocated_blocks(blocks);
+    if (e == cudaSuccess) e = launch_reset(dv_, blocks.list, blocks.count, stream_);
     mark_end(kKReset);
     if (e == cudaSuccess) e = cudaMemsetAsync(counters_, 0, sizeof(VolumeCounters), stream_);
     // Every completed update leaves the per-voxel batch state at zero, so it is

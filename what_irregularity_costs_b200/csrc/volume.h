@@ -216,10 +216,14 @@ private:
     cudaError_t run_update(const BatchArgs& a, const UpdateScratch& u, bool insert,
                            const FrameTable* frames = nullptr, const PoseTable* poses = nullptr);
     bool ensure_records(int64_t n_records);
-    // The allocated blocks' pool indices: 0..n-1 in the pool layout (returns
-    // nullptr), the occupied slots listed on the device in the slot-index
-    // layout (returns the list; n = block count).
-    const int32_t* block_list(int32_t n);
+    // The allocated blocks, counted on the device: pool indices
+    // 0..*count-1 in the pool layout (list: nullptr), the occupied slots listed
+    // by a kernel in the slot-index layout.
+    struct Blocks {
+        const int32_t* list;
+        const int32_t* count;
+    };
+    cudaError_t allocated_blocks(Blocks& out);
     int32_t* block_list_ = nullptr;  // slot-index layout: [pool] occupied slots
     int32_t* list_count_ = nullptr;
     bool ensure_mesh(int32_t cap, bool rgb);
@@ -253,7 +257,8 @@ private:
     float* mesh_posnor_ = nullptr;
     uint8_t* mesh_rgb_ = nullptr;
     int32_t mesh_cap_ = 0;
-    int32_t* mesh_ctl_ = nullptr;  // [0] vertex count, [1] overflow flag
+    static constexpr int kMeshCounters = 3;
+    int32_t* mesh_ctl_ = nullptr;  // [0] vertex count, [1] overflow flag, [2] blocks handed out
     FrameCam* d_frames_ = nullptr;  // frame table of the last several-frame integrate
     FramePose* d_poses_ = nullptr;  // poses of the last several-image depth integrate
 
@@ -307,9 +312,10 @@ size_t voxel_arrays(int storage, const DevVolume& d, void* out[5], size_t bytes[
 cudaError_t launch_reset(const DevVolume& v, const int32_t* list, const int32_t* count, cudaStream_t s);
 // List the occupied slots of the table (slot-index layout) into out.
 cudaError_t launch_list_blocks(const DevVolume& v, int32_t* out, int32_t* count, cudaStream_t s);
-// Extraction over n blocks: pool indices 0..n-1, or those of a list.
-cudaError_t launch_extract(const DevVolume& v, int32_t n_blocks, const int32_t* list, float min_w, float iso,
-                           float* posnor, uint8_t* rgb, int32_t cap, int32_t* ctl, cudaStream_t s);
+// Extraction over the allocated blocks: pool indices 0..*count-1, or the
+// *count entries of a list (count: device memory).
+cudaError_t launch_extract(const DevVolume& v, const int32_t* list, const int32_t* count, float min_w, float iso,
+                           float* posnor, uint8_t* rgb, int32_t cap, int32_t* ctl, int sm_count, cudaStream_t s);
 
 // The update pipeline: band walk (counts, sums, records) -> finish -> group
 // (grouping, ordered selection and finishing of the voxels that cross the cap).
