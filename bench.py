@@ -632,9 +632,9 @@ def run_ours(args):
         hist += vol.allocate_probe_histogram(d_all[a:b], cams[k], n_bins=32)
     probes_mean = float(np.sum(hist * np.arange(32)) / max(1, int(hist.sum())))
     integrate_kernels = ("band", "finish", "group", "select")
-    # Launches of the headline arm: per integrate_frames call the set-up
-    # kernel and the four passes; reset's two per step.
-    launches_per_step = (1 + sum(1 for k in integrate_kernels if per_kernel[k][1] > 0)) * len(groups) + 2
+    # Launches of the headline arm: the four passes of every integrate_frames
+    # call and the reset kernel, per step.
+    launches_per_step = sum(1 for k in integrate_kernels if per_kernel[k][1] > 0) * len(groups) + 1
     dominant = max(integrate_kernels, key=lambda k: per_kernel[k][0])
 
     peak, peak_kind = measured_peak()

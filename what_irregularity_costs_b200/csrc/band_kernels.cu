@@ -38,8 +38,8 @@
 // so leaving them out changes no result.
 //
 // Several frames per call (band_frames_kernel, band_depth_frames_kernel): the
-// same walk, each point seen from the camera of its frame (a per-call table
-// the set-up kernel stores; depth images also carry their poses). The points
+// same walk, each point seen from the camera of its frame (a table among the
+// kernel's parameters; depth images also carry their poses). The points
 // of frame k precede those of frame k+1, so the canonical (point, step) order
 // is (frame, point, step) order and the cap keeps what per-frame calls keep.
 #include <algorithm>
@@ -67,15 +67,7 @@ constexpr int kBandMinBlocks = OSN_BAND_MIN_BLOCKS;
 
 // Band records and slot values are read once more, by the group pass of the
 // same update: stored with the streaming hint (1, evict-first) or as
-// ordinary write-back stores that may stay in L2 (0).
-// 1: a several-frame walk is launched with programmatic stream serialisation
-// behind its one-CTA set-up kernel, so its CTAs are resident when the set-up
-// ends (they wait for it on the device; measured 0.8 % faster on the room
-// trajectory); 0: an ordinary launch.
-#ifndef OSN_BAND_PDL
-#define OSN_BAND_PDL 1
-#endif
-
+// ordinary write-back stores that may stay in L2 (0; no difference measured).
 #ifndef OSN_BAND_STREAM_RECORDS
 #define OSN_BAND_STREAM_RECORDS 1
 #endif
@@ -595,17 +587,15 @@ struct OneCamera {
 // only move forward (tile += grid size), so its frame does too: one
 // comparison per tile, and a table read only where the frame changes.
 struct FrameCursor {
-    const FrameCam* frames;
-    int32_t n, f, next;
+    const FrameTable& table;  // kernel parameter
+    int32_t f, next;
     float cx, cy, cz;
-    __device__ __forceinline__ FrameCursor(const FrameCam* fr, int32_t nf) : frames(fr), n(nf), f(0) {
-        load();
-    }
+    __device__ __forceinline__ explicit FrameCursor(const FrameTable& t) : table(t), f(0) { load(); }
     __device__ __forceinline__ void load() {
-        cx = __ldg(&frames[f].x);
-        cy = __ldg(&frames[f].y);
-        cz = __ldg(&frames[f].z);
-        next = f + 1 < n ? __ldg(&frames[f + 1].begin) : INT_MAX;
+        cx = table.f[f].x;
+        cy = table.f[f].y;
+        cz = table.f[f].z;
+        next = f + 1 < table.n ? table.f[f + 1].begin : INT_MAX;
     }
     __device__ __forceinline__ void at(int i) {
         while (i >= next) {  // the last frame's bound is INT_MAX
@@ -685,9 +675,13 @@ __device__ __forceinline__ void band_tiles(const DevVolume& v, const BatchArgs& 
     if (t == 0 && s_counted) atomicAdd(&u.ctl->n_records, (int)s_counted);
 }
 
+// Every walk is launched with programmatic stream serialisation: its CTAs take
+// their places while the previous call's last pass drains, and wait here for
+// what that call wrote.
 template <int MODE, bool RECORDS, int S, bool DEPTH = false>
 __global__ void __launch_bounds__(kBandThreads, kBandMinBlocks)
 band_kernel(DevVolume v, BatchArgs a, UpdateScratch u, unsigned long long* hist, int n_bins) {
+    grid_dependency_wait();
     band_tiles<MODE, RECORDS, S, false>(v, a, u, hist, n_bins, BatchPoints<DEPTH ? 1 : 0>{a}, OneCamera{});
 }
 
@@ -695,52 +689,25 @@ band_kernel(DevVolume v, BatchArgs a, UpdateScratch u, unsigned long long* hist,
 // single-frame walk with each point's camera taken from the frame table.
 template <int S>
 __global__ void __launch_bounds__(kBandThreads, kBandMinBlocks)
-band_frames_kernel(DevVolume v, BatchArgs a, UpdateScratch u, const FrameCam* frames, int32_t n_frames) {
-    if (OSN_BAND_PDL) grid_dependency_wait();  // the set-up kernel's frame table and zeroed counters
-    band_tiles<kAllocInsert, true, S, true>(v, a, u, nullptr, 0, BatchPoints<0>{a}, FrameCursor(frames, n_frames));
+band_frames_kernel(DevVolume v, BatchArgs a, UpdateScratch u, const __grid_constant__ FrameTable frames) {
+    grid_dependency_wait();
+    band_tiles<kAllocInsert, true, S, true>(v, a, u, nullptr, 0, BatchPoints<0>{a}, FrameCursor(frames));
 }
 
 // The same for several depth images of equal size: each CTA stages the
 // images' poses in shared memory first.
 template <int S>
 __global__ void __launch_bounds__(kBandThreads, kBandMinBlocks)
-band_depth_frames_kernel(DevVolume v, BatchArgs a, UpdateScratch u, const FrameCam* frames,
-                         const FramePose* poses, int32_t n_frames) {
+band_depth_frames_kernel(DevVolume v, BatchArgs a, UpdateScratch u, const __grid_constant__ FrameTable frames,
+                         const __grid_constant__ PoseTable poses) {
     __shared__ FramePose s_pose[kMaxDepthFrames];
-    if (OSN_BAND_PDL) grid_dependency_wait();  // the set-up kernel's tables and zeroed counters
     constexpr int kWords = (int)(sizeof(FramePose) / sizeof(double));
-    for (int k = threadIdx.x; k < n_frames * kWords; k += blockDim.x)
-        reinterpret_cast<double*>(s_pose)[k] = __ldg(reinterpret_cast<const double*>(poses) + k);
+    for (int k = threadIdx.x; k < poses.n * kWords; k += blockDim.x)
+        reinterpret_cast<double*>(s_pose)[k] = reinterpret_cast<const double*>(poses.p)[k];
+    grid_dependency_wait();
     __syncthreads();
-    band_tiles<kAllocInsert, true, S, true>(v, a, u, nullptr, 0, DepthFramesPoints{a, s_pose, a.n / n_frames},
-                                            FrameCursor(frames, n_frames));
-}
-
-// Set-up of a several-frame integrate, in place of the control block's
-// memset: zero the control block and store the frame table where the band
-// walk reads it (one CTA; static indices only, so the table stays in the
-// parameter space).
-__global__ void frames_setup_kernel(UpdateControl* ctl, FrameCam* dst, const FrameTable t) {
-    if (OSN_BAND_PDL) launch_dependents();  // the walk's CTAs may take their places now
-    const int k = threadIdx.x;
-    if (k < (int)(sizeof(UpdateControl) / sizeof(uint32_t))) reinterpret_cast<uint32_t*>(ctl)[k] = 0u;
-#pragma unroll
-    for (int j = 0; j <= kMaxFrames; ++j)
-        if (j == k && j <= t.n) dst[j] = t.f[j];
-}
-
-// The same for several depth images, with their poses.
-__global__ void frames_setup_depth_kernel(UpdateControl* ctl, FrameCam* dst, const FrameTable t,
-                                          FramePose* pdst, const PoseTable p) {
-    if (OSN_BAND_PDL) launch_dependents();
-    const int k = threadIdx.x;
-    if (k < (int)(sizeof(UpdateControl) / sizeof(uint32_t))) reinterpret_cast<uint32_t*>(ctl)[k] = 0u;
-#pragma unroll
-    for (int j = 0; j <= kMaxFrames; ++j)
-        if (j == k && j <= t.n) dst[j] = t.f[j];
-#pragma unroll
-    for (int j = 0; j < kMaxDepthFrames; ++j)
-        if (j == k && j < p.n) pdst[j] = p.p[j];
+    band_tiles<kAllocInsert, true, S, true>(v, a, u, nullptr, 0, DepthFramesPoints{a, s_pose, a.n / poses.n},
+                                            FrameCursor(frames));
 }
 
 // ---- batched steps -----------------------------------------------------
@@ -855,8 +822,7 @@ cudaError_t launch(const DevVolume& v, const BatchArgs& a, const UpdateScratch& 
     });
     const int tiles = (a.n + kBandThreads - 1) / kBandThreads;
     const int grid = std::min(tiles, per_sm * sm_count);
-    band_kernel<MODE, RECORDS, S, DEPTH><<<grid, kBandThreads, 0, s>>>(v, a, u, hist, n_bins);
-    return cudaGetLastError();
+    return launch_after(band_kernel<MODE, RECORDS, S, DEPTH>, grid, kBandThreads, s, v, a, u, hist, n_bins);
 }
 
 }  // namespace
@@ -905,7 +871,7 @@ cudaError_t launch_band_records(const DevVolume& v, const BatchArgs& a, const Up
 namespace {
 template <int S>
 cudaError_t launch_band_frames_t(const DevVolume& v, const BatchArgs& a, const UpdateScratch& u,
-                                 const FrameCam* frames, int32_t n_frames, int sm_count, cudaStream_t s) {
+                                 const FrameTable& frames, int sm_count, cudaStream_t s) {
     static int per_sm = 0;
     static std::once_flag once;
     std::call_once(once, [] {
@@ -916,14 +882,12 @@ cudaError_t launch_band_frames_t(const DevVolume& v, const BatchArgs& a, const U
     });
     const int tiles = (a.n + kBandThreads - 1) / kBandThreads;
     const int grid = std::min(tiles, per_sm * sm_count);
-    if (OSN_BAND_PDL) return launch_after(band_frames_kernel<S>, grid, kBandThreads, s, v, a, u, frames, n_frames);
-    band_frames_kernel<S><<<grid, kBandThreads, 0, s>>>(v, a, u, frames, n_frames);
-    return cudaGetLastError();
+    return launch_after(band_frames_kernel<S>, grid, kBandThreads, s, v, a, u, frames);
 }
 template <int S>
 cudaError_t launch_band_depth_frames_t(const DevVolume& v, const BatchArgs& a, const UpdateScratch& u,
-                                       const FrameCam* frames, const FramePose* poses, int32_t n_frames,
-                                       int sm_count, cudaStream_t s) {
+                                       const FrameTable& frames, const PoseTable& poses, int sm_count,
+                                       cudaStream_t s) {
     static int per_sm = 0;
     static std::once_flag once;
     std::call_once(once, [] {
@@ -934,43 +898,26 @@ cudaError_t launch_band_depth_frames_t(const DevVolume& v, const BatchArgs& a, c
     });
     const int tiles = (a.n + kBandThreads - 1) / kBandThreads;
     const int grid = std::min(tiles, per_sm * sm_count);
-    if (OSN_BAND_PDL)
-        return launch_after(band_depth_frames_kernel<S>, grid, kBandThreads, s, v, a, u, frames, poses, n_frames);
-    band_depth_frames_kernel<S><<<grid, kBandThreads, 0, s>>>(v, a, u, frames, poses, n_frames);
-    return cudaGetLastError();
+    return launch_after(band_depth_frames_kernel<S>, grid, kBandThreads, s, v, a, u, frames, poses);
 }
 }  // namespace
 
-cudaError_t launch_frames_setup(UpdateControl* ctl, FrameCam* d_frames, const FrameTable& t, cudaStream_t s) {
-    frames_setup_kernel<<<1, 64, 0, s>>>(ctl, d_frames, t);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_frames_setup_depth(UpdateControl* ctl, FrameCam* d_frames, const FrameTable& t,
-                                      FramePose* d_poses, const PoseTable& p, cudaStream_t s) {
-    frames_setup_depth_kernel<<<1, 64, 0, s>>>(ctl, d_frames, t, d_poses, p);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_band_depth_frames(const DevVolume& v, const BatchArgs& a, const UpdateScratch& u,
-                                     const FrameCam* d_frames, const FramePose* d_poses, int32_t n_frames,
-                                     int sm_count, cudaStream_t s) {
-    if (a.n <= 0 || n_frames < 1 || n_frames > kMaxDepthFrames || a.n % n_frames != 0)
-        return cudaErrorInvalidValue;
+                                     const FrameTable& frames, const PoseTable& poses, int sm_count, cudaStream_t s) {
+    if (a.n <= 0 || poses.n < 1 || poses.n > kMaxDepthFrames || a.n % poses.n != 0) return cudaErrorInvalidValue;
     switch (v.storage) {
-        case kStoreF32: return launch_band_depth_frames_t<kStoreF32>(v, a, u, d_frames, d_poses, n_frames, sm_count, s);
-        case kStoreF16U16:
-            return launch_band_depth_frames_t<kStoreF16U16>(v, a, u, d_frames, d_poses, n_frames, sm_count, s);
+        case kStoreF32: return launch_band_depth_frames_t<kStoreF32>(v, a, u, frames, poses, sm_count, s);
+        case kStoreF16U16: return launch_band_depth_frames_t<kStoreF16U16>(v, a, u, frames, poses, sm_count, s);
         default: return cudaErrorInvalidValue;
     }
 }
 
 cudaError_t launch_band_frames(const DevVolume& v, const BatchArgs& a, const UpdateScratch& u,
-                               const FrameCam* d_frames, int32_t n_frames, int sm_count, cudaStream_t s) {
+                               const FrameTable& frames, int sm_count, cudaStream_t s) {
     if (a.n <= 0) return cudaSuccess;
     switch (v.storage) {
-        case kStoreF32: return launch_band_frames_t<kStoreF32>(v, a, u, d_frames, n_frames, sm_count, s);
-        case kStoreF16U16: return launch_band_frames_t<kStoreF16U16>(v, a, u, d_frames, n_frames, sm_count, s);
+        case kStoreF32: return launch_band_frames_t<kStoreF32>(v, a, u, frames, sm_count, s);
+        case kStoreF16U16: return launch_band_frames_t<kStoreF16U16>(v, a, u, frames, sm_count, s);
         default: return cudaErrorInvalidValue;  // the FP64 oracle integrates one frame per batch
     }
 }

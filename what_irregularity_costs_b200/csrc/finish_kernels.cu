@@ -299,6 +299,8 @@ finish_kernel(DevVolume v, UpdateScratch u) {
     __syncthreads();
     launch_dependents();
     grid_dependency_wait();
+    if (u.next_ctl && blockIdx.x == 0 && t < (int)(sizeof(UpdateControl) / sizeof(uint32_t)))
+        reinterpret_cast<uint32_t*>(u.next_ctl)[t] = 0u;  // for the next update; its last user is done
     const int n_touched = min(u.ctl->n_touched, v.pool_capacity);
     int updated = 0;
     for (int ia = blockIdx.x; ia < n_touched; ia += 2 * gridDim.x) {

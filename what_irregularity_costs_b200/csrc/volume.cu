@@ -101,7 +101,7 @@ bool Volume::alloc_device(uint32_t hash_slots) {
     OSN_TRY(cudaMalloc(&us_.vacc, n_vox * sizeof(unsigned long long)));
     OSN_TRY(cudaMalloc(&us_.xbits, (size_t)dv_.pool_capacity * kXWords * sizeof(uint32_t)));
     OSN_TRY(cudaMalloc(&us_.touched, (size_t)dv_.pool_capacity * sizeof(int32_t)));
-    OSN_TRY(cudaMalloc(&us_.ctl, sizeof(UpdateControl)));
+    OSN_TRY(cudaMalloc(&us_.ctl, 2 * sizeof(UpdateControl)));
     us_.status = dv_.status;
     OSN_TRY(cudaMalloc(&mesh_ctl_, kMeshCounters * sizeof(int32_t)));
     if (dv_.slot_index) {
@@ -126,7 +126,7 @@ bool Volume::alloc_device(uint32_t hash_slots) {
     OSN_TRY(cudaMemsetAsync(us_.vcnt, 0, n_vox * sizeof(uint32_t), stream_));
     OSN_TRY(cudaMemsetAsync(us_.vacc, 0, n_vox * sizeof(unsigned long long), stream_));
     OSN_TRY(cudaMemsetAsync(us_.xbits, 0, (size_t)dv_.pool_capacity * kXWords * sizeof(uint32_t), stream_));
-    OSN_TRY(cudaMemsetAsync(us_.ctl, 0, sizeof(UpdateControl), stream_));
+    OSN_TRY(cudaMemsetAsync(us_.ctl, 0, 2 * sizeof(UpdateControl), stream_));
     OSN_TRY(cudaStreamSynchronize(stream_));
     return true;
 }
@@ -157,8 +157,6 @@ Volume::~Volume() {
     cudaFree(mesh_ctl_);
     cudaFree(block_list_);
     cudaFree(list_count_);
-    cudaFree(d_frames_);
-    cudaFree(d_poses_);
     if (host_small_) cudaFreeHost(host_small_);
     for (auto& p : pending_) {
         cudaEventDestroy(p.start);
@@ -296,6 +294,7 @@ bool Volume::set_pipelined(bool on) {
     synchronize();
     if (!on) {
         pipelined_ = false;
+        if (last_ctl_ == us2_.ctl) last_ctl_ = nullptr;  // its set goes
         free_second_set();
         for (int k = 0; k < 2; ++k) {
             if (band_done_[k]) cudaEventDestroy(band_done_[k]);
@@ -304,7 +303,6 @@ bool Volume::set_pipelined(bool on) {
         }
         if (tail_) cudaStreamDestroy(tail_);
         tail_ = nullptr;
-        if (last_ctl_ != us_.ctl && last_ctl_ != nullptr) last_ctl_ = nullptr;  // its set is gone
         return true;
     }
     if (dv_.storage == kStoreF64) return false;  // the oracle's tail reads the points
@@ -359,14 +357,18 @@ cudaError_t Volume::run_update(const BatchArgs& a, const UpdateScratch& scratch,
     unfinished_ = true;  // until every pass of this update is queued
     cudaError_t e = cudaSuccess;
     if (pipe) e = cudaStreamWaitEvent(stream_, tail_done_[p], 0);
-    if (e == cudaSuccess)
-        e = poses    ? launch_frames_setup_depth(u.ctl, d_frames_, *frames, d_poses_, *poses, stream_)
-            : frames ? launch_frames_setup(u.ctl, d_frames_, *frames, stream_)
-                     : cudaMemsetAsync(u.ctl, 0, sizeof(UpdateControl), stream_);
+    bool clear = true;
+    if (!pipelined_ && scratch.ctl == us_.ctl) {
+        u.ctl = us_.ctl + ctl_turn_;
+        u.next_ctl = us_.ctl + (ctl_turn_ ^ 1);
+        clear = !ctl_clear_;
+    }
+    ctl_clear_ = false;  // until every pass of this update is queued
+    if (e == cudaSuccess && clear) e = cudaMemsetAsync(u.ctl, 0, sizeof(UpdateControl), stream_);
     if (e != cudaSuccess) return e;
     mark_start(kKBand);
-    e = poses    ? launch_band_depth_frames(dv_, a, u, d_frames_, d_poses_, frames->n, sm_count_, stream_)
-        : frames ? launch_band_frames(dv_, a, u, d_frames_, frames->n, sm_count_, stream_)
+    e = poses    ? launch_band_depth_frames(dv_, a, u, *frames, *poses, sm_count_, stream_)
+        : frames ? launch_band_frames(dv_, a, u, *frames, sm_count_, stream_)
                  : launch_band_records(dv_, a, u, insert, sm_count_, stream_);
     mark_end(kKBand);
     if (e != cudaSuccess) return e;
@@ -379,19 +381,25 @@ cudaError_t Volume::run_update(const BatchArgs& a, const UpdateScratch& scratch,
     e = launch_finish(dv_, u, sm_count_, tail);
     mark_end(kKFinish, tail);
     if (e != cudaSuccess) return e;
-    mark_start(kKGroup, tail);
-    e = launch_group(dv_, a, u, sm_count_, tail);
-    mark_end(kKGroup, tail);
-    if (e != cudaSuccess) return e;
-    mark_start(kKSelect, tail);
-    e = launch_select(dv_, a, u, sm_count_, tail);
-    mark_end(kKSelect, tail);
-    if (e != cudaSuccess) return e;
+    if (dv_.weight_cap > 0.0f) {  // without a cap no voxel crosses it
+        mark_start(kKGroup, tail);
+        e = launch_group(dv_, a, u, sm_count_, tail);
+        mark_end(kKGroup, tail);
+        if (e != cudaSuccess) return e;
+        mark_start(kKSelect, tail);
+        e = launch_select(dv_, a, u, sm_count_, tail);
+        mark_end(kKSelect, tail);
+        if (e != cudaSuccess) return e;
+    }
     if (pipe) {
         if ((e = cudaEventRecord(tail_done_[p], tail_)) != cudaSuccess) return e;
         ++n_updates_;
     }
     unfinished_ = was_unfinished;
+    if (u.next_ctl) {
+        ctl_turn_ ^= 1;
+        ctl_clear_ = true;
+    }
     return cudaSuccess;
 }
 
@@ -411,14 +419,6 @@ cudaError_t Volume::integrate(const BatchArgs& a) {
 cudaError_t Volume::integrate_frames(const BatchArgs& a, const FrameTable& t, const PoseTable* poses) {
     if (dv_.storage == kStoreF64) return cudaErrorInvalidValue;  // one frame per oracle batch
     if ((poses != nullptr) != (a.depth.depth != nullptr)) return cudaErrorInvalidValue;
-    if (!d_frames_ && cudaMalloc(&d_frames_, sizeof(FrameCam) * (kMaxFrames + 1)) != cudaSuccess) {
-        d_frames_ = nullptr;
-        return cudaErrorMemoryAllocation;
-    }
-    if (poses && !d_poses_ && cudaMalloc(&d_poses_, sizeof(FramePose) * kMaxDepthFrames) != cudaSuccess) {
-        d_poses_ = nullptr;
-        return cudaErrorMemoryAllocation;
-    }
     if (!ensure_records(batch_records(a.n, dv_.steps))) return cudaErrorMemoryAllocation;
     return run_update(a, us_, true, &t, poses);
 }
@@ -501,6 +501,7 @@ SceneWork Volume::batch_work(const BatchArgs& a, cudaStream_t s) {
     w.a = a;
     w.u = us_;
     w.u.tag = update_tag_;
+    ctl_clear_ = false;  // the step uses the first control block
     w.band_tiles = (a.n + kBatchTilePoints - 1) / kBatchTilePoints;
     w.n_slots = (int32_t)batch_records(a.n, dv_.steps);
     return w;

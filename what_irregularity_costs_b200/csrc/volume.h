@@ -27,8 +27,10 @@ enum KernelId : int {
     kNumKernelIds = 8,
 };
 
-// Counters an update pass keeps on the device (one small struct, cleared by
-// one memset at the start of every update).
+// Counters an update keeps on the device, zero when it starts. Serial updates
+// take two control blocks in turn: each update's finish pass clears the other
+// one for the next (a memset of its own before every walk cost 2-3 us a call).
+// Pipelined, batched and no-alloc updates clear theirs first.
 struct UpdateControl {
     int32_t n_records;   // band records counted (contributions that can be accepted)
     int32_t n_touched;   // blocks that received a band sample
@@ -79,6 +81,7 @@ struct PoseTable {
 
 struct UpdateScratch {
     UpdateControl* ctl = nullptr;
+    UpdateControl* next_ctl = nullptr;  // cleared by the finish pass (null: nothing to clear)
     uint32_t* records = nullptr;  // [record_cap] one per band slot
     float* slot_val = nullptr;    // [record_cap] normalised SDF of each counted slot (FP32 / FP16
                                   // storage; null for the FP64 oracle, which recomputes it)
@@ -248,6 +251,10 @@ private:
     cudaEvent_t band_done_[2] = {nullptr, nullptr};
     cudaEvent_t tail_done_[2] = {nullptr, nullptr};
     uint64_t n_updates_ = 0;
+    // Serial updates: which of the two control blocks at us_.ctl is next, and
+    // whether the last update has cleared it.
+    int ctl_turn_ = 0;
+    bool ctl_clear_ = false;
     UpdateControl* last_ctl_ = nullptr;  // counters of the last update
     bool alloc_second_set();
     void free_second_set();
@@ -259,8 +266,6 @@ private:
     int32_t mesh_cap_ = 0;
     static constexpr int kMeshCounters = 3;
     int32_t* mesh_ctl_ = nullptr;  // [0] vertex count, [1] overflow flag, [2] blocks handed out
-    FrameCam* d_frames_ = nullptr;  // frame table of the last several-frame integrate
-    FramePose* d_poses_ = nullptr;  // poses of the last several-image depth integrate
 
     // Pinned host staging for small reads.
     int64_t* host_small_ = nullptr;
@@ -321,18 +326,13 @@ cudaError_t launch_extract(const DevVolume& v, const int32_t* list, const int32_
 // (grouping, ordered selection and finishing of the voxels that cross the cap).
 cudaError_t launch_band_records(const DevVolume& v, const BatchArgs& a, const UpdateScratch& u,
                                 bool insert, int sm_count, cudaStream_t s);
-// Several-frame integrate: the set-up kernel (control block zeroed, frame
-// table stored) and the band walk with per-frame cameras (FP32 / FP16 storage).
-cudaError_t launch_frames_setup(UpdateControl* ctl, FrameCam* d_frames, const FrameTable& t, cudaStream_t s);
+// Several-frame integrate: the walk with per-frame cameras (FP32 / FP16 storage).
 cudaError_t launch_band_frames(const DevVolume& v, const BatchArgs& a, const UpdateScratch& u,
-                               const FrameCam* d_frames, int32_t n_frames, int sm_count, cudaStream_t s);
-// The same for depth images (a.depth set): poses stored by the set-up, the
-// walk unprojecting image i / (width * height) with its pose.
-cudaError_t launch_frames_setup_depth(UpdateControl* ctl, FrameCam* d_frames, const FrameTable& t,
-                                      FramePose* d_poses, const PoseTable& p, cudaStream_t s);
+                               const FrameTable& frames, int sm_count, cudaStream_t s);
+// The same for depth images (a.depth set): the walk unprojects image
+// i / (width * height) with its pose.
 cudaError_t launch_band_depth_frames(const DevVolume& v, const BatchArgs& a, const UpdateScratch& u,
-                                     const FrameCam* d_frames, const FramePose* d_poses, int32_t n_frames,
-                                     int sm_count, cudaStream_t s);
+                                     const FrameTable& frames, const PoseTable& poses, int sm_count, cudaStream_t s);
 cudaError_t launch_finish(const DevVolume& v, const UpdateScratch& u, int sm_count, cudaStream_t s);
 cudaError_t launch_group(const DevVolume& v, const BatchArgs& a, const UpdateScratch& u, int sm_count,
                          cudaStream_t s);
