@@ -84,7 +84,7 @@ def test_walk_drops_where_the_pool_is_full(cuda):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("n", [1, 7, 29, 257, 2051])
-@pytest.mark.parametrize("cap", [1.0, 5.0])
+@pytest.mark.parametrize("cap", [1.0, 2.5, 5.0])
 def test_every_record_crosses(cuda, n, cap):
     """Grouping where all 256 band slots of a warp belong to cap-crossing
     voxels, and where the slots end inside a thread's eight."""

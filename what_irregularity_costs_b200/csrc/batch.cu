@@ -278,7 +278,7 @@ private:
     cudaError_t passes(const StepWork& w, const BatchShape& shape) {
         cudaError_t e = launch_batch_prepare(w, stream_);
         if (e == cudaSuccess) e = launch_band_multi(w, storage_, sm_count_, stream_);
-        if (e == cudaSuccess) e = launch_finish_multi(w, storage_, shape.finish_pair, sm_count_, stream_);
+        if (e == cudaSuccess) e = launch_finish_multi(w, storage_, sm_count_, stream_);
         if (e == cudaSuccess) e = launch_group_multi(w, storage_, sm_count_, stream_);
         if (e == cudaSuccess) e = launch_select_multi(w, storage_, sm_count_, stream_);
         return e;

@@ -20,7 +20,8 @@
 // the fixed-point sum of the records' normalised SDFs, the list of touched
 // blocks, and per band slot a record (the voxel) and the normalised SDF.
 //
-//   finish   one 128-thread CTA per touched block (two per CTA pass), 4
+//   finish   one 128-thread CTA per touched block, the next block's counts
+//            and the next but one's index read ahead, 4
 //            voxels per thread, every array read and written as 128-bit
 //            vectors: a voxel that accepts all of its records (keep == n,
 //            the common case) gets tsdf + sum, w0 + n, 128 * (w0 + n) and
@@ -70,7 +71,8 @@ constexpr int kSelectWarps = kSelectThreads / 32;
 #ifndef OSN_GROUP_MIN_BLOCKS
 #define OSN_GROUP_MIN_BLOCKS 6
 #endif
-static_assert(kFinishThreads >= kMaxBatchScenes && kGroupThreads >= kMaxBatchScenes,
+static_assert(kFinishThreads >= kMaxBatchScenes && kGroupThreads >= kMaxBatchScenes &&
+                  kSelectThreads >= kMaxBatchScenes,
               "one thread per scene builds the item prefix");
 
 // Contributions a voxel accepts given its weight w0 before the batch and n
@@ -80,11 +82,41 @@ __device__ __forceinline__ int accept_count(float w0, float cap, int n) {
     if (n == 0) return 0;
     if (!(cap > 0.0f)) return n;
     if (w0 >= cap) return 0;
+    // Room for all of them (the common case), exact where weight and count
+    // are integers below 2^23.
+    if (w0 < 8388608.0f && n < (1 << 23) && __fadd_rn(w0, (float)(n - 1)) < cap) return n;
     const double room = ceil((double)cap - (double)w0);
     return room >= (double)n ? n : (int)room;
 }
 
 // ---- finish ----------------------------------------------------------------
+
+// What finishing a volume's touched blocks reads and writes.
+struct FinishArgs {
+    float* tsdf;
+    float* weight;
+    float* r;
+    float* g;
+    float* b;
+    uint32_t* vcnt;
+    unsigned long long* vacc;
+    uint32_t* xbits;
+    uint32_t* xlist;
+    const int32_t* touched;
+    UpdateControl* ctl;
+    uint32_t* status;
+    int32_t* block_chunk;
+    uint32_t record_cap, xlist_cap;  // places (32-bit in the control block too)
+    float cap;                       // effective weight cap
+    int32_t chunk;
+};
+
+__device__ __forceinline__ FinishArgs finish_args(const DevVolume& v, const UpdateScratch& u) {
+    constexpr int64_t kMost = 0xFFFFFFFF;
+    return FinishArgs{v.tsdf, v.weight, v.r, v.g, v.b, u.vcnt, u.vacc, u.xbits, u.xlist, u.touched, u.ctl, v.status,
+                      v.block_chunk, (uint32_t)min(u.record_cap, (int64_t)kMost), (uint32_t)min(u.xlist_cap, (int64_t)kMost),
+                      v.weight_cap, v.chunk};
+}
 
 // Four consecutive voxels of one storage mode, as registers.
 template <int S>
@@ -95,7 +127,7 @@ struct Quad {
 };
 
 template <int S>
-__device__ __forceinline__ void load_quad(const DevVolume& v, size_t q4, Quad<S>& x) {
+__device__ __forceinline__ void load_quad(const FinishArgs& v, size_t q4, Quad<S>& x) {
     if constexpr (S == kStoreF32) {
         const float4 w4 = reinterpret_cast<const float4*>(v.weight)[q4];
         const float4 t4 = reinterpret_cast<const float4*>(v.tsdf)[q4];
@@ -119,7 +151,7 @@ __device__ __forceinline__ void load_quad(const DevVolume& v, size_t q4, Quad<S>
 }
 
 template <int S>
-__device__ __forceinline__ void store_quad(const DevVolume& v, size_t q4, const Quad<S>& x) {
+__device__ __forceinline__ void store_quad(const FinishArgs& v, size_t q4, const Quad<S>& x) {
     if constexpr (S == kStoreF32) {
         reinterpret_cast<float4*>(v.tsdf)[q4] = make_float4(x.t[0], x.t[1], x.t[2], x.t[3]);
         reinterpret_cast<float4*>(v.weight)[q4] = make_float4(x.w[0], x.w[1], x.w[2], x.w[3]);
@@ -152,7 +184,10 @@ __device__ __forceinline__ void store_quad(const DevVolume& v, size_t q4, const 
 //            (the caller rounds);
 //   FP64: the double sum.
 __device__ __forceinline__ float new_mean_f16(float mean0, float w0, int keep, long long fix) {
-    const float sum = __fadd_rn(__fmul_rn(mean0, w0), (float)((double)fix * kFixInv));
+    // (float)((double)fix * 2^-40); one conversion where the double is exact.
+    const bool exact = fix > -(1ll << 53) && fix < (1ll << 53);
+    const float add = exact ? __fmul_rn(__ll2float_rn(fix), (float)kFixInv) : (float)((double)fix * kFixInv);
+    const float sum = __fadd_rn(__fmul_rn(mean0, w0), add);
     return __fdiv_rn(sum, __fadd_rn(w0, (float)keep));
 }
 
@@ -177,17 +212,26 @@ __device__ __forceinline__ void cta_add(int* smem_acc, int mine, int* global) {
     if (threadIdx.x == 0 && *smem_acc) atomicAdd(global, *smem_acc);
 }
 
-// One touched block's quad of voxels, its arrays already loaded: finish
-// the voxels that accept all their records, open groups for those that
-// cross the cap. Warp-synchronous (all lanes of the warp call it).
+// Thread t's four voxels of touched block bi, their batch counts c4 already
+// loaded: finish the voxels that accept all their records, open groups for
+// those that cross the cap. The other arrays are read only where a count is
+// set (in about a third of a touched block). Warp-synchronous (all lanes of the
+// warp call it).
 template <int S>
-__device__ __forceinline__ void finish_quad(const DevVolume& v, const UpdateScratch& u, int32_t bi,
-                                            size_t q4, int t, int lane, const uint4 c4, Quad<S>& x,
-                                            const ulonglong2 a01, const ulonglong2 a23, int& updated) {
+__device__ __forceinline__ void finish_quad(const FinishArgs& f, int32_t bi, int t, int lane, const uint4 c4,
+                                            int& updated) {
     const bool any = (c4.x | c4.y | c4.z | c4.w) != 0u;
     // Warp-uniform skip: no record of this update names these 128 voxels, so
     // the group pass never reads their crossing bits either.
     if (!__any_sync(0xffffffffu, any)) return;
+    const size_t q4 = (size_t)bi * (kBlockVoxels / 4) + t;
+    Quad<S> x{};
+    ulonglong2 a01 = make_ulonglong2(0ull, 0ull), a23 = a01;
+    if (any) {
+        load_quad<S>(f, q4, x);
+        a01 = reinterpret_cast<const ulonglong2*>(f.vacc)[2 * q4];
+        a23 = reinterpret_cast<const ulonglong2*>(f.vacc)[2 * q4 + 1];
+    }
     const uint32_t n[4] = {c4.x, c4.y, c4.z, c4.w};
     unsigned long long acc[4] = {a01.x, a01.y, a23.x, a23.y};
     uint32_t cnt[4] = {0u, 0u, 0u, 0u};
@@ -198,7 +242,7 @@ __device__ __forceinline__ void finish_quad(const DevVolume& v, const UpdateScra
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         if (n[q] == 0u) continue;
-        keepv[q] = accept_count(x.w[q], v.weight_cap, (int)n[q]);
+        keepv[q] = accept_count(x.w[q], f.cap, (int)n[q]);
         if (keepv[q] != 0 && (uint32_t)keepv[q] != n[q]) {
             my_records += n[q];
             ++my_cross;
@@ -217,8 +261,8 @@ __device__ __forceinline__ void finish_quad(const DevVolume& v, const UpdateScra
         }
         uint32_t rb = 0u, xb = 0u;
         if (lane == 31) {
-            rb = atomicAdd(&u.ctl->x_used, rec_incl);
-            xb = (uint32_t)atomicAdd(&u.ctl->n_crossing, (unsigned long long)x_incl);
+            rb = atomicAdd(&f.ctl->x_used, rec_incl);
+            xb = (uint32_t)atomicAdd(&f.ctl->n_crossing, (unsigned long long)x_incl);
         }
         rb = __shfl_sync(0xffffffffu, rb, 31);
         xb = __shfl_sync(0xffffffffu, xb, 31);
@@ -241,16 +285,16 @@ __device__ __forceinline__ void finish_quad(const DevVolume& v, const UpdateScra
             // last of them finishes it. The sum word holds the group's base
             // + 1 (high half) and the next free place (low half); the count
             // word the records still to be placed.
-            if ((uint64_t)rec_base + n[q] <= (uint64_t)u.record_cap && x_at < (uint32_t)u.xlist_cap) {
+            if ((uint64_t)rec_base + n[q] <= (uint64_t)f.record_cap && x_at < f.xlist_cap) {
                 acc[q] = (unsigned long long)(rec_base + 1u) << 32;
                 cnt[q] = n[q];
                 xmask |= 1u << q;
-                u.xlist[x_at] = (uint32_t)bi * kBlockVoxels + 4u * t + q;
+                f.xlist[x_at] = (uint32_t)bi * kBlockVoxels + 4u * t + q;
             } else {
                 // Out of scratch (only after a failed update left stale
                 // counters): the voxel's records are dropped, the status
                 // word says so.
-                atomicOr(v.status, kStatusScratchOverflow);
+                atomicOr(f.status, kStatusScratchOverflow);
                 acc[q] = 0ull;
             }
             rec_base += n[q];
@@ -263,38 +307,69 @@ __device__ __forceinline__ void finish_quad(const DevVolume& v, const UpdateScra
     bits |= __shfl_xor_sync(0xffffffffu, bits, 1);
     bits |= __shfl_xor_sync(0xffffffffu, bits, 2);
     bits |= __shfl_xor_sync(0xffffffffu, bits, 4);
-    if ((t & 7) == 0) u.xbits[(size_t)bi * kXWords + (t >> 3)] = bits;
+    if ((t & 7) == 0) f.xbits[(size_t)bi * kXWords + (t >> 3)] = bits;
     if (!any) return;
-    store_quad<S>(v, q4, x);
-    reinterpret_cast<uint4*>(u.vcnt)[q4] = make_uint4(cnt[0], cnt[1], cnt[2], cnt[3]);
-    reinterpret_cast<ulonglong2*>(u.vacc)[2 * q4] = make_ulonglong2(acc[0], acc[1]);
-    reinterpret_cast<ulonglong2*>(u.vacc)[2 * q4 + 1] = make_ulonglong2(acc[2], acc[3]);
+    store_quad<S>(f, q4, x);
+    reinterpret_cast<uint4*>(f.vcnt)[q4] = make_uint4(cnt[0], cnt[1], cnt[2], cnt[3]);
+    reinterpret_cast<ulonglong2*>(f.vacc)[2 * q4] = make_ulonglong2(acc[0], acc[1]);
+    reinterpret_cast<ulonglong2*>(f.vacc)[2 * q4 + 1] = make_ulonglong2(acc[2], acc[3]);
 }
 
-// A touched block now belongs to the current call's chunk.
-__device__ __forceinline__ void tag_chunk(const DevVolume& v, int32_t ba, int32_t bb, bool has_b) {
-    if (!v.block_chunk) return;
-    v.block_chunk[ba] = v.chunk;
-    if (has_b) v.block_chunk[bb] = v.chunk;
+// Touched blocks first, first + stride, ... < n, one per pass of the CTA. A
+// pass needs three dependent reads (the block's index, its counts, its other
+// arrays); the index of the next but one block and the counts of the next are
+// read ahead, so a pass waits for one of them. Blocks come from a source of
+// one or several scenes: seek(sc, i) is item i's scene (at or after sc).
+// done(sc, updated) takes the voxels this thread rewrote.
+template <int S, typename Source, typename Done>
+__device__ __forceinline__ void finish_stream(int first, int n, int stride, const Source& src, const Done& done) {
+    const int t = threadIdx.x, lane = t & 31;
+    const auto counts = [&](int i, int sc, int32_t bi) {
+        return i < n ? reinterpret_cast<const uint4*>(src.args(sc).vcnt)[(size_t)bi * (kBlockVoxels / 4) + t]
+                     : make_uint4(0u, 0u, 0u, 0u);
+    };
+    const auto seek = [&](int sc, int i) { return i < n ? src.seek(sc, i) : sc; };
+    const auto index = [&](int i, int sc) { return i < n ? src.touched(sc, i) : 0; };
+    int sc = seek(0, first), sc1 = seek(sc, first + stride);
+    int32_t bi = index(first, sc), bi1 = index(first + stride, sc1);
+    uint4 c4 = counts(first, sc, bi);
+    for (int i = first; i < n; i += stride) {
+        const uint4 c1 = counts(i + stride, sc1, bi1);
+        const int sc2 = seek(sc1, i + 2 * stride);
+        const int32_t bi2 = index(i + 2 * stride, sc2);
+        const FinishArgs& f = src.args(sc);
+        if (t == 0 && f.block_chunk) f.block_chunk[bi] = f.chunk;  // the block now belongs to the call's chunk
+        int updated = 0;
+        finish_quad<S>(f, bi, t, lane, c4, updated);
+        done(sc, updated);
+        sc = sc1;
+        sc1 = sc2;
+        bi = bi1;
+        bi1 = bi2;
+        c4 = c1;
+    }
 }
 
+struct OneVolumeBlocks {
+    const FinishArgs& f;
+    __device__ __forceinline__ int seek(int, int) const { return 0; }
+    __device__ __forceinline__ const FinishArgs& args(int) const { return f; }
+    __device__ __forceinline__ int32_t touched(int, int i) const { return f.touched[i]; }
+};
+
+// Resident CTAs per SM the registers are sized for: 8 (64 registers). One
+// 640x480 frame takes 16.7 us either way at 8 and 10; twelve batched scenes 4.93
+// ms at 8, 5.36 at 10 (spills), 5.67 at 7. Packing the counted voxels so that
+// sparse warps run full was slower on FP32 storage (28.7 us against 20.6 on
+// four frames: eight 4-byte accesses a voxel instead of 16-byte ones).
+#ifndef OSN_FINISH_MIN_BLOCKS
+#define OSN_FINISH_MIN_BLOCKS 8
+#endif
 template <int S>
-__device__ __forceinline__ void load_item(const DevVolume& v, const UpdateScratch& u, size_t q4,
-                                          uint4& c4, Quad<S>& x, ulonglong2& a01, ulonglong2& a23) {
-    c4 = reinterpret_cast<const uint4*>(u.vcnt)[q4];
-    load_quad<S>(v, q4, x);
-    a01 = reinterpret_cast<const ulonglong2*>(u.vacc)[2 * q4];
-    a23 = reinterpret_cast<const ulonglong2*>(u.vacc)[2 * q4 + 1];
-}
-
-// Two touched blocks per CTA iteration: the indices of both, then every
-// array of both, are in flight together (each CTA pass is two dependent
-// round trips, whatever the number of blocks it covers).
-template <int S>
-__global__ void __launch_bounds__(kFinishThreads)
+__global__ void __launch_bounds__(kFinishThreads, S == kStoreF64 ? 1 : OSN_FINISH_MIN_BLOCKS)
 finish_kernel(DevVolume v, UpdateScratch u) {
     __shared__ int s_updated;
-    const int t = threadIdx.x, lane = t & 31;
+    const int t = threadIdx.x;
     if (t == 0) s_updated = 0;
     __syncthreads();
     launch_dependents();
@@ -302,24 +377,11 @@ finish_kernel(DevVolume v, UpdateScratch u) {
     if (u.next_ctl && blockIdx.x == 0 && t < (int)(sizeof(UpdateControl) / sizeof(uint32_t)))
         reinterpret_cast<uint32_t*>(u.next_ctl)[t] = 0u;  // for the next update; its last user is done
     const int n_touched = min(u.ctl->n_touched, v.pool_capacity);
-    int updated = 0;
-    for (int ia = blockIdx.x; ia < n_touched; ia += 2 * gridDim.x) {
-        const int ib = ia + gridDim.x;
-        const bool has_b = ib < n_touched;  // uniform across the CTA
-        const int32_t ba = u.touched[ia];
-        const int32_t bb = has_b ? u.touched[ib] : ba;
-        const size_t qa = (size_t)ba * (kBlockVoxels / 4) + t;  // this thread's 4 voxels
-        const size_t qb = (size_t)bb * (kBlockVoxels / 4) + t;
-        uint4 ca, cb;
-        Quad<S> xa, xb;
-        ulonglong2 a01, a23, b01, b23;
-        load_item<S>(v, u, qa, ca, xa, a01, a23);
-        if (has_b) load_item<S>(v, u, qb, cb, xb, b01, b23);
-        if (t == 0) tag_chunk(v, ba, bb, has_b);
-        finish_quad<S>(v, u, ba, qa, t, lane, ca, xa, a01, a23, updated);
-        if (has_b) finish_quad<S>(v, u, bb, qb, t, lane, cb, xb, b01, b23, updated);
-    }
-    cta_add(&s_updated, updated, &u.ctl->n_updated);
+    const FinishArgs f = finish_args(v, u);
+    int sum = 0;
+    finish_stream<S>((int)blockIdx.x, n_touched, (int)gridDim.x, OneVolumeBlocks{f},
+                     [&](int, int updated) { sum += updated; });
+    cta_add(&s_updated, sum, &u.ctl->n_updated);
 }
 
 // ---- group and select ------------------------------------------------------
@@ -829,7 +891,7 @@ __global__ void batch_prepare_kernel(StepWork w) {
 
 // Work items a pass has in one scene (read by thread 0 after the previous
 // pass completed).
-enum MultiPass : int { kPassFinishPairs, kPassFinishSingle, kPassGroup, kPassSelect };
+enum MultiPass : int { kPassFinish, kPassGroup, kPassSelect };
 
 template <int PASS>
 __device__ __forceinline__ int scene_items(const SceneWork& sw) {
@@ -837,15 +899,9 @@ __device__ __forceinline__ int scene_items(const SceneWork& sw) {
     // counters (and an empty batch): it has no work in any pass.
     if (sw.band_tiles <= 0) return 0;
     const UpdateControl* c = sw.u.ctl;
-    if (PASS == kPassFinishPairs || PASS == kPassFinishSingle) {
-        const int nt = min(c->n_touched, sw.v.pool_capacity);
-        return PASS == kPassFinishPairs ? (nt + 1) / 2 : nt;
-    }
+    if (PASS == kPassFinish) return min(c->n_touched, sw.v.pool_capacity);
     if (c->n_crossing == 0ull) return 0;  // no voxel crossed the cap in this scene
-    if (PASS == kPassSelect) {
-        const long long x = min((long long)c->n_crossing, (long long)sw.u.xlist_cap);
-        return (int)(sw.v.storage == kStoreF64 ? x : (x + kSelectChunk - 1) / kSelectChunk);  // voxels, or chunks
-    }
+    if (PASS == kPassSelect) return (int)min((long long)c->n_crossing, (long long)sw.u.xlist_cap);
     return (int)(((uint32_t)sw.n_slots + kGroupThreads * kGroupPerThread - 1) /
                  (kGroupThreads * kGroupPerThread));
 }
@@ -864,61 +920,42 @@ __device__ __forceinline__ void scene_prefix(const StepWork& w, int* begin) {
     __syncthreads();
 }
 
-// Finish every touched block of every scene: work items of one or two
-// blocks from an atomic queue, the item's scene descriptor staged in shared
-// memory (reloaded when the CTA moves to another scene).
-template <int S, bool PAIR>
-__global__ void __launch_bounds__(kFinishThreads)
+// Finish every touched block of every scene: the scenes' blocks as one list,
+// dealt out evenly (290 us a step on twelve scenes from a queue, with a barrier
+// and five dependent round trips an item; 180 so); the scenes' arguments in
+// shared memory.
+struct SceneBlocks {
+    const FinishArgs* scene;
+    const int* begin;
+    __device__ __forceinline__ int seek(int sc, int i) const {
+        while (i >= begin[sc + 1]) ++sc;
+        return sc;
+    }
+    __device__ __forceinline__ const FinishArgs& args(int sc) const { return scene[sc]; }
+    __device__ __forceinline__ int32_t touched(int sc, int i) const { return scene[sc].touched[i - begin[sc]]; }
+};
+
+template <int S>
+__global__ void __launch_bounds__(kFinishThreads, S == kStoreF64 ? 1 : OSN_FINISH_MIN_BLOCKS)
 finish_multi_kernel(StepWork w) {
-    __shared__ SceneWork sw;
+    __shared__ FinishArgs s_args[kMaxBatchScenes];
     __shared__ int s_begin[kMaxBatchScenes + 1];
-    __shared__ int s_item, s_updated;
-    const int t = threadIdx.x, lane = t & 31;
+    __shared__ int s_updated[kMaxBatchScenes];
+    const int t = threadIdx.x;
     launch_dependents();
     grid_dependency_wait();
-    if (t == 0) s_updated = 0;
-    scene_prefix<PAIR ? kPassFinishPairs : kPassFinishSingle>(w, s_begin);
-    const int total = s_begin[w.n_scenes];
-    int cur = -1, updated = 0;
-    for (;;) {
-        if (t == 0) s_item = (int)atomicAdd(&w.queues[kQFinish], 1u);
-        __syncthreads();
-        const int item = s_item;
-        const bool done = item >= total;  // also on a CTA's first pull when items are few
-        const int sc = done ? -1 : scene_of(s_begin, w.n_scenes, item);
-        if (sc != cur || done) {
-            // Statistics of the scene left behind, then the next descriptor.
-            const int wsum = __reduce_add_sync(0xffffffffu, updated);
-            if (lane == 0 && wsum) atomicAdd(&s_updated, wsum);
-            __syncthreads();
-            if (t == 0 && cur >= 0 && s_updated) atomicAdd(&sw.u.ctl->n_updated, s_updated);
-            __syncthreads();
-            if (t == 0) s_updated = 0;
-            updated = 0;
-            if (done) break;
-            cta_copy(&sw, &w.scenes[sc]);
-            __syncthreads();
-            cur = sc;
-        }
-        const int n_touched = min(sw.u.ctl->n_touched, sw.v.pool_capacity);
-        const int local = item - s_begin[sc];
-        const int ia = PAIR ? 2 * local : local;
-        const int ib = ia + 1;
-        const bool has_b = PAIR && ib < n_touched;  // uniform across the CTA
-        const int32_t ba = sw.u.touched[ia];
-        const int32_t bb = has_b ? sw.u.touched[ib] : ba;
-        const size_t qa = (size_t)ba * (kBlockVoxels / 4) + t;
-        const size_t qb = (size_t)bb * (kBlockVoxels / 4) + t;
-        uint4 ca, cb;
-        Quad<S> xa, xb;
-        ulonglong2 a01, a23, b01, b23;
-        load_item<S>(sw.v, sw.u, qa, ca, xa, a01, a23);
-        if (has_b) load_item<S>(sw.v, sw.u, qb, cb, xb, b01, b23);
-        if (t == 0) tag_chunk(sw.v, ba, bb, has_b);
-        finish_quad<S>(sw.v, sw.u, ba, qa, t, lane, ca, xa, a01, a23, updated);
-        if (has_b) finish_quad<S>(sw.v, sw.u, bb, qb, t, lane, cb, xb, b01, b23, updated);
-        __syncthreads();  // s_item and the descriptor are rewritten next
+    if (t < w.n_scenes) {
+        s_args[t] = finish_args(w.scenes[t].v, w.scenes[t].u);
+        s_updated[t] = 0;
     }
+    scene_prefix<kPassFinish>(w, s_begin);
+    finish_stream<S>((int)blockIdx.x, s_begin[w.n_scenes], (int)gridDim.x, SceneBlocks{s_args, s_begin},
+                     [&](int sc, int updated) {
+                         const int sum = __reduce_add_sync(0xffffffffu, updated);
+                         if ((t & 31) == 0 && sum) atomicAdd(&s_updated[sc], sum);
+                     });
+    __syncthreads();
+    if (t < w.n_scenes && s_updated[t]) atomicAdd(&s_args[t].ctl->n_updated, s_updated[t]);
 }
 
 // Group, select and finish the cap-crossing voxels of every scene that has
@@ -955,33 +992,42 @@ group_multi_kernel(StepWork w) {
     }
 }
 
-// The ordered selection of every scene's cap-crossing voxels: warp work
-// items, one per listed voxel.
+// The ordered selection of every scene's cap-crossing voxels. Each scene gets
+// warps in proportion to its voxels, and a warp takes every so-manieth voxel of
+// its scene's list, as in one volume: neighbours in the list are neighbours in
+// a block, whose groups are large together (32 consecutive voxels per warp from
+// a queue took 170 us a step on twelve scenes, against 75).
 template <int S>
-__global__ void __launch_bounds__(kSelectThreads)
+__global__ void __launch_bounds__(kSelectThreads, S == kStoreF64 ? 1 : 5)
 select_multi_kernel(StepWork w) {
     __shared__ uint32_t hist[kSelectWarps][256];
-    __shared__ int s_begin[kMaxBatchScenes + 1];
+    __shared__ int s_count[kMaxBatchScenes];      // listed voxels of each scene
+    __shared__ int s_begin[kMaxBatchScenes + 1];  // warps before each scene
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     launch_dependents();
     grid_dependency_wait();
-    scene_prefix<kPassSelect>(w, s_begin);
-    const int total = s_begin[w.n_scenes];
-    for (;;) {
-        int item = 0;
-        if (lane == 0) item = (int)atomicAdd(&w.queues[kQSelect], 1u);
-        item = __shfl_sync(0xffffffffu, item, 0);
-        if (item >= total) break;
+    const int nw = (int)gridDim.x * kSelectWarps;
+    if ((int)threadIdx.x < w.n_scenes) s_count[threadIdx.x] = scene_items<kPassSelect>(w.scenes[threadIdx.x]);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        long long total = 0;
+        for (int k = 0; k < w.n_scenes; ++k) total += s_count[k];
+        const long long per = max(1ll, (total + nw - 1) / nw);  // voxels a warp
+        s_begin[0] = 0;
+        for (int k = 0; k < w.n_scenes; ++k) s_begin[k + 1] = s_begin[k] + (int)((s_count[k] + per - 1) / per);
+    }
+    __syncthreads();
+    for (int item = (int)blockIdx.x * kSelectWarps + warp; item < s_begin[w.n_scenes]; item += nw) {
         const int sc = scene_of(s_begin, w.n_scenes, item);
         const SceneWork& sw = w.scenes[sc];
         const SelectArgs sa = select_args(sw.v, sw.u);
-        int done;
+        const long long n = s_count[sc], step = s_begin[sc + 1] - s_begin[sc];
+        int done = 0;
         if constexpr (S == kStoreF64) {
-            done = select_group<S>(sa, sw.v, sw.a, sw.u.xlist[item - s_begin[sc]], hist[warp], lane);
+            for (long long d = item - s_begin[sc]; d < n; d += step)
+                done += select_group<S>(sa, sw.v, sw.a, sw.u.xlist[d], hist[warp], lane);
         } else {
-            const long long n = min((long long)sw.u.ctl->n_crossing, (long long)sw.u.xlist_cap);
-            const long long c0 = (long long)kSelectChunk * (item - s_begin[sc]);
-            done = select_stream<S>(sa, sw.u.xlist, c0, min(n, c0 + kSelectChunk), 1, hist[warp], lane);
+            done = select_stream<S>(sa, sw.u.xlist, item - s_begin[sc], n, step, hist[warp], lane);
         }
         done = __reduce_add_sync(0xffffffffu, done);
         if (lane == 0 && done) atomicAdd(&sw.u.ctl->n_updated, done);
@@ -1055,10 +1101,9 @@ cudaError_t launch_batch_prepare(const StepWork& w, cudaStream_t s) {
 }
 
 namespace {
-template <int S, bool P>
+template <int S>
 cudaError_t finish_multi_t(const StepWork& w, int sm_count, cudaStream_t s) {
-    return launch_after(finish_multi_kernel<S, P>,
-                        resident_grid<finish_multi_kernel<S, P>>(kFinishThreads, sm_count),
+    return launch_after(finish_multi_kernel<S>, resident_grid<finish_multi_kernel<S>>(kFinishThreads, sm_count),
                         kFinishThreads, s, w);
 }
 template <int S>
@@ -1073,17 +1118,11 @@ cudaError_t group_multi_t(const StepWork& w, int sm_count, cudaStream_t s) {
 }
 }  // namespace
 
-cudaError_t launch_finish_multi(const StepWork& w, int storage, int pair, int sm_count, cudaStream_t s) {
+cudaError_t launch_finish_multi(const StepWork& w, int storage, int sm_count, cudaStream_t s) {
     switch (storage) {
-        case kStoreF16U16:
-            return pair ? finish_multi_t<kStoreF16U16, true>(w, sm_count, s)
-                        : finish_multi_t<kStoreF16U16, false>(w, sm_count, s);
-        case kStoreF64:
-            return pair ? finish_multi_t<kStoreF64, true>(w, sm_count, s)
-                        : finish_multi_t<kStoreF64, false>(w, sm_count, s);
-        default:
-            return pair ? finish_multi_t<kStoreF32, true>(w, sm_count, s)
-                        : finish_multi_t<kStoreF32, false>(w, sm_count, s);
+        case kStoreF16U16: return finish_multi_t<kStoreF16U16>(w, sm_count, s);
+        case kStoreF64: return finish_multi_t<kStoreF64>(w, sm_count, s);
+        default: return finish_multi_t<kStoreF32>(w, sm_count, s);
     }
 }
 

@@ -484,7 +484,7 @@ __device__ __forceinline__ long long to_fix(float x) { return __float2ll_rn(x * 
 __device__ __forceinline__ long long to_fix(double x) { return __double2ll_rn(x * kFixScale); }
 
 __device__ __forceinline__ float add_fix(float t0, long long sum) {
-    return __double2float_rn((double)t0 + (double)sum * kFixInv);
+    return __double2float_rn(__fma_rn((double)sum, kFixInv, (double)t0));  // the product is exact
 }
 
 // Programmatic dependent launch. A kernel launched with programmatic stream

@@ -363,13 +363,13 @@ struct SceneWork {
 };
 
 // Work queues of one step, one counter per pass (zeroed by the prepare pass).
-enum BatchQueue : int { kQBand = 0, kQFinish, kQGroup, kQSelect, kNumBatchQueues };
+enum BatchQueue : int { kQBand = 0, kQGroup, kNumBatchQueues };
 
 // Tunable shape of a batched step (chosen by the batch autotuner).
 struct BatchShape {
     int band_tiles_per_item = 4;  // band work item: this many 128-point tiles of one scene
     int probe = 0;                // accepted (0 or 1); the walk has one resolution scheme now
-    int finish_pair = 1;          // finish work item: 1 = two touched blocks, 0 = one
+    int finish_pair = 1;          // accepted (0 or 1); finish deals its blocks out evenly now
 };
 
 // Everything a batched pass reads: the scene table and the queues.
@@ -383,7 +383,7 @@ struct StepWork {
 
 cudaError_t launch_batch_prepare(const StepWork& w, cudaStream_t s);
 cudaError_t launch_band_multi(const StepWork& w, int storage, int sm_count, cudaStream_t s);
-cudaError_t launch_finish_multi(const StepWork& w, int storage, int pair, int sm_count, cudaStream_t s);
+cudaError_t launch_finish_multi(const StepWork& w, int storage, int sm_count, cudaStream_t s);
 cudaError_t launch_group_multi(const StepWork& w, int storage, int sm_count, cudaStream_t s);
 cudaError_t launch_select_multi(const StepWork& w, int storage, int sm_count, cudaStream_t s);
 
