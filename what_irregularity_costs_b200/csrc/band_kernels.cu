@@ -6,8 +6,8 @@
 // :259-269, :302-337 (one thread per point, one hash probe sequence per
 // sample).
 //
-// One thread walks one point's band (2*steps+1 samples, kChunk at a time in
-// registers); a persistent grid of CTAs strides over tiles of 128
+// One thread walks one point's band (2*steps+1 samples, kChunk at a time, in its
+// columns of shared memory); a persistent grid of CTAs strides over tiles of 128
 // consecutive points (neighbouring pixels of a frame). The blocks of a warp's
 // samples are resolved through a small table in shared memory (band_point):
 // every distinct block of the 32 points is probed once, by one lane, with all
@@ -17,9 +17,10 @@
 //
 // What bounds it (four 640x480 frames a call): L1 throughput of the scattered
 // weight gathers and reductions (about 21 M sectors, one a cycle per SM: 75
-// us) and instruction issue (53.6 M warp instructions: 48 us); 122 us
-// measured, 143 before the table (67.1 M instructions, and values spilled
-// around calls).
+// us) and instruction issue (53 M warp instructions: 48 us); 105 us measured.
+// 143 before the table (67 M instructions, and values spilled around calls);
+// 121 with the samples in registers, whose columns left room for fewer loads in
+// flight than shared memory does.
 //
 // Update tail. The resolving lane also tags the block as touched by this update
 // (one atomic exchange on the spare word of its table slot, unless the probe
@@ -56,14 +57,18 @@ static_assert(kBandThreads >= kMaxBatchScenes, "one thread per scene builds the 
 #ifndef OSN_BAND_CHUNK
 #define OSN_BAND_CHUNK 9
 #endif
-constexpr int kChunk = OSN_BAND_CHUNK;  // samples per ray held in registers (9: the whole band at 4 voxels)
-// Resident CTAs per SM the register budget is sized for: 6 (80 registers,
-// nothing spilled). Four 640x480 frames per call took 121 us at 6, 124 at 7
-// (72 registers), 131 at 8 (64); one frame 43.8 us at 6, 44.9 at 8.
+constexpr int kChunk = OSN_BAND_CHUNK;  // samples per ray walked together (9: the whole band at 4 voxels)
+// Resident CTAs per SM the register budget is sized for. Four 640x480 frames
+// per call took 104.7 us at 7 (72 registers), 106.5 at 6 and 8, 115.6 at 9; one
+// frame 39.4 us at 8 (64 registers), 40.8 at 6 and 7.
 #ifndef OSN_BAND_MIN_BLOCKS
-#define OSN_BAND_MIN_BLOCKS 6
+#define OSN_BAND_MIN_BLOCKS 8
+#endif
+#ifndef OSN_BAND_FRAMES_MIN_BLOCKS
+#define OSN_BAND_FRAMES_MIN_BLOCKS 7
 #endif
 constexpr int kBandMinBlocks = OSN_BAND_MIN_BLOCKS;
+constexpr int kBandFramesMinBlocks = OSN_BAND_FRAMES_MIN_BLOCKS;
 
 // Band records and slot values are read once more, by the group pass of the
 // same update: stored with the streaming hint (1, evict-first) or as
@@ -207,49 +212,55 @@ __device__ __forceinline__ void red_add(unsigned long long* p, unsigned long lon
 // Shared memory of one band CTA.
 //   table    per warp: the blocks of its samples (x: key within the warp, y:
 //            pool index)
+//   vox      per thread: its samples' voxel offsets, then their voxels
+//   dsq      per thread: its samples' squared distances
 //   run_key  measurement modes: per-thread columns of run keys (x: low word),
 //            run q of thread t at [q][t] (no bank conflicts)
 constexpr int kTableEntries = 64;  // two per lane
 template <bool MEASURE>
 struct BandSmem {
     uint2 table[MEASURE ? 1 : kBandThreads / 32][kTableEntries];
+    uint32_t vox[MEASURE ? 1 : kChunk][kBandThreads];
+    float dsq[MEASURE ? 1 : kChunk][kBandThreads];
     uint2 run_key[MEASURE ? kChunk : 1][kBandThreads];
 };
 
 // N consecutive band samples of a ray once their blocks are resolved: the
 // voxels' weights gathered together, then the saturation gate, counts, sums
-// and records. vox: the samples' voxels or kNoVoxel; dsq: squared distance of
-// camera and voxel centre (unfused float arithmetic, as the reference's), from
-// which the signed distance is taken only where a lane counts; f64: the FP64
-// oracle's value of sample j. n_steps: samples in use (warp-uniform). writes:
-// this lane's records are stored.
+// and records. vox, dsq: this thread's columns of the samples' voxels (or
+// kNoVoxel) and squared distances of camera and voxel centre (unfused float
+// arithmetic, as the reference's), from which the signed distance is taken only
+// where a lane counts; f64: the FP64 oracle's value of sample j. n_steps:
+// samples in use (warp-uniform). writes: this lane's records are stored.
 template <int S, int N, typename F64>
 __device__ __forceinline__ void count_samples(const DevVolume& v, const UpdateScratch& u, bool writes,
-                                              uint32_t stride, float dist, uint32_t (&vox)[N],
-                                              const float (&dsq)[N], int n_steps, uint32_t& slot,
-                                              uint32_t& counted, const F64& f64) {
+                                              uint32_t stride, float dist, const uint32_t* vox, const float* dsq,
+                                              int n_steps, uint32_t& slot, uint32_t& counted, const F64& f64) {
     // Without a cap no voxel can be full or cross it: no weight is looked at,
     // and no record is kept for the cap selection.
     const bool capped = v.weight_cap > 0.0f;
+    uint32_t at[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) at[j] = j < n_steps ? vox[j * kBandThreads] : kNoVoxel;
     if (capped) {
         float w0[N];
 #pragma unroll
-        for (int j = 0; j < N; ++j) w0[j] = weight_at<S>(v, vox[j] == kNoVoxel ? 0u : vox[j]);
+        for (int j = 0; j < N; ++j) w0[j] = weight_at<S>(v, at[j] == kNoVoxel ? 0u : at[j]);
 #pragma unroll
         for (int j = 0; j < N; ++j)
-            if (w0[j] >= v.weight_cap) vox[j] = kNoVoxel;  // takes no contribution
+            if (w0[j] >= v.weight_cap) at[j] = kNoVoxel;  // takes no contribution
     }
 #pragma unroll
     for (int j = 0; j < N; ++j) {
         if (j >= n_steps) break;
-        const bool counts = vox[j] != kNoVoxel;
+        const bool counts = at[j] != kNoVoxel;
         if (__any_sync(0xffffffffu, counts)) {
             long long fix;
             float sdf_n = 0.0f;
             if constexpr (S == kStoreF64) {
                 fix = counts ? f64(j) : 0ll;
             } else {
-                const float sdf = __fsub_rn(dist, __fsqrt_rn(dsq[j]));
+                const float sdf = __fsub_rn(dist, __fsqrt_rn(dsq[j * kBandThreads]));
                 sdf_n = fminf(fmaxf(__fmul_rn(sdf, v.inv_trunc), -1.0f), 1.0f);
                 fix = to_fix(sdf_n);
             }
@@ -257,12 +268,12 @@ __device__ __forceinline__ void count_samples(const DevVolume& v, const UpdateSc
                 // Kept for the records of voxels that cross the cap, so the
                 // update tail never reads the batch's points again.
                 if (S != kStoreF64 && capped) store_slot(u.slot_val + slot, sdf_n);
-                red_add(&u.vcnt[vox[j]], 1u);
-                red_add(&u.vacc[vox[j]], (unsigned long long)fix);
+                red_add(&u.vcnt[at[j]], 1u);
+                red_add(&u.vacc[at[j]], (unsigned long long)fix);
                 ++counted;
             }
         }
-        if (capped && writes) store_slot(u.records + slot, vox[j]);  // read again by the group pass
+        if (capped && writes) store_slot(u.records + slot, at[j]);  // read again by the group pass
         slot += stride;
     }
 }
@@ -432,33 +443,34 @@ __device__ __forceinline__ void band_point(const DevVolume& v, const BatchArgs& 
             table[lane].x = kNoOffset;
             table[lane + 32].x = kNoOffset;
             __syncwarp();
-            uint32_t vox[kChunk];  // voxel offset, then the voxel's index
-            float dsq[kChunk];
+            uint32_t* const vox = &sm.vox[0][threadIdx.x];  // voxel offset, then the voxel's index
+            float* const dsq = &sm.dsq[0][threadIdx.x];
 #pragma unroll
             for (int j = 0; j < kChunk; ++j) {
-                const float t = __fmul_rn((float)c0 + (float)j, v.voxel_size);
+                if (j >= n_steps) break;
+                const float t = __fmul_rn((float)(c0 + j), v.voxel_size);
                 const float yx = __fadd_rd(__fmul_rn(__fadd_rn(px, __fmul_rn(r.ux, t)), v.inv_voxel), kFloorMagic);
                 const float yy = __fadd_rd(__fmul_rn(__fadd_rn(py, __fmul_rn(r.uy, t)), v.inv_voxel), kFloorMagic);
                 const float yz = __fadd_rd(__fmul_rn(__fadd_rn(pz, __fmul_rn(r.uz, t)), v.inv_voxel), kFloorMagic);
                 const float ex = __fsub_rn(__fmaf_rn(__fsub_rn(yx, kFloorMagic), v.voxel_size, half), cx);
                 const float ey = __fsub_rn(__fmaf_rn(__fsub_rn(yy, kFloorMagic), v.voxel_size, half), cy);
                 const float ez = __fsub_rn(__fmaf_rn(__fsub_rn(yz, kFloorMagic), v.voxel_size, half), cz);
-                dsq[j] = __fadd_rn(__fadd_rn(__fmul_rn(ex, ex), __fmul_rn(ey, ey)), __fmul_rn(ez, ez));
+                const float d2 = __fadd_rn(__fadd_rn(__fmul_rn(ex, ex), __fmul_rn(ey, ey)), __fmul_rn(ez, ez));
                 const uint32_t w = pack_offset(__float_as_uint(yx), __float_as_uint(yy), __float_as_uint(yz)) - base;
-                bool ok = mine && j < n_steps;
-                if (c0 + j > sure_step) ok = ok && !(__fsub_rn(r.dist, __fsqrt_rn(dsq[j])) < -v.trunc);
-                vox[j] = ok ? w : kNoOffset;
+                bool ok = mine;
+                if (c0 + j > sure_step) ok = ok && !(__fsub_rn(r.dist, __fsqrt_rn(d2)) < -v.trunc);
+                vox[j * kBandThreads] = ok ? w : kNoOffset;
+                // The oracle's value needs the voxel's offset.
+                dsq[j * kBandThreads] = S == kStoreF64 ? __uint_as_float(w) : d2;
                 if (ok) table[table_entry(w)].x = w & kOffsetBlock;
             }
             __syncwarp();
 
-            bool met = false;
-            unsigned done = 0u;  // once met: bit j, sample j has its voxel
+            unsigned done = 0u;  // bit j: sample j has its voxel
             for (;;) {
                 // The blocks in the table, one or two per lane. A slot's 16
                 // bytes hold the key, the index and the touch tag.
-                bool dropped = false;
-#pragma unroll
+#pragma unroll 1
                 for (int k = 0; k < kTableEntries / 32; ++k) {
                     const uint32_t b = table[lane + 32 * k].x;
                     const bool need = b != kNoOffset;
@@ -479,57 +491,37 @@ __device__ __forceinline__ void band_point(const DevVolume& v, const BatchArgs& 
                     __syncwarp();
                     if (RECORDS) tag_touched<false>(v, u, res.bi >= 0 && (rest || seen != u.tag), res.bi, res.slot);
                     if (need) table[lane + 32 * k].y = (uint32_t)res.bi;
-                    dropped |= need && res.bi < 0;
                 }
                 __syncwarp();
-                if (!met) {
-                    // Every sample's entry, all loads in flight together, no branch.
-                    bool miss = false;
-                    uint32_t at[kChunk];
-#pragma unroll
-                    for (int j = 0; j < kChunk; ++j) {
-                        const uint2 e = table[table_entry(vox[j])];
-                        const bool hit = e.x == (vox[j] & kOffsetBlock);
-                        miss |= !hit && vox[j] != kNoOffset;
-                        at[j] = hit ? __funnelshift_l(voxel_high(vox[j]), e.y, 9) : kNoVoxel;
-                        // The oracle's value needs the voxel's offset.
-                        if constexpr (S == kStoreF64) dsq[j] = __uint_as_float(vox[j]);
-                    }
-                    if (!__any_sync(0xffffffffu, miss || dropped)) {
-#pragma unroll
-                        for (int j = 0; j < kChunk; ++j) vox[j] = at[j];
-                        break;
-                    }
-                }
-                // Two blocks met in an entry (met: further rounds for the
-                // samples left), or a block was dropped.
-                met = true;
                 bool left = false;
 #pragma unroll
                 for (int j = 0; j < kChunk; ++j) {
-                    if (vox[j] == kNoOffset || ((done >> j) & 1u)) continue;
-                    const uint2 e = table[table_entry(vox[j])];
-                    if (e.x != (vox[j] & kOffsetBlock)) {
-                        left = true;
-                        continue;
+                    const uint32_t w = j < n_steps ? vox[j * kBandThreads] : kNoOffset;
+                    const uint2 e = table[table_entry(w)];
+                    const bool open = w != kNoOffset && !((done >> j) & 1u), hit = open && e.x == (w & kOffsetBlock);
+                    left |= open && !hit;
+                    if (hit) {
+                        done |= 1u << j;
+                        if (counts_drops && (int)e.y < 0) ++drops;
+                        vox[j * kBandThreads] = (int)e.y < 0 ? kNoVoxel : __funnelshift_l(voxel_high(w), e.y, 9);
                     }
-                    done |= 1u << j;
-                    if (counts_drops && (int)e.y < 0) ++drops;
-                    vox[j] = (int)e.y < 0 ? kNoVoxel : __funnelshift_l(voxel_high(vox[j]), e.y, 9);
                 }
                 if (!__any_sync(0xffffffffu, left)) break;
+                // Two blocks met in an entry: another round for the samples left.
                 __syncwarp();
                 table[lane].x = kNoOffset;
                 table[lane + 32].x = kNoOffset;
                 __syncwarp();
-#pragma unroll
-                for (int j = 0; j < kChunk; ++j)
-                    if (vox[j] != kNoOffset && !((done >> j) & 1u)) table[table_entry(vox[j])].x = vox[j] & kOffsetBlock;
+#pragma unroll 1
+                for (int j = 0; j < n_steps; ++j) {
+                    const uint32_t w = vox[j * kBandThreads];
+                    if (w != kNoOffset && !((done >> j) & 1u)) table[table_entry(w)].x = w & kOffsetBlock;
+                }
                 __syncwarp();
             }
             if (RECORDS)
-                count_samples<S>(v, u, writes, (uint32_t)a.n, r.dist, vox, dsq, n_steps, slot, counted, [&](int j) {
-                    const uint32_t w = __float_as_uint(dsq[j]);
+                count_samples<S, kChunk>(v, u, writes, (uint32_t)a.n, r.dist, vox, dsq, n_steps, slot, counted, [&](int j) {
+                    const uint32_t w = __float_as_uint(dsq[j * kBandThreads]);
                     return oracle_fix(v, a, r, (int)(ox - kFloorBits + (w & 2047u)),
                                       (int)(oy - kFloorBits + ((w >> 11) & 2047u)), (int)(oz - kFloorBits + (w >> 22)));
                 });
@@ -548,8 +540,8 @@ __device__ __forceinline__ void band_point(const DevVolume& v, const BatchArgs& 
 #pragma unroll 1
     for (int s = -v.steps; s <= v.steps; ++s) {
         int vx = 0, vy = 0, vz = 0;
-        float dsq[1] = {0.0f};
-        const bool ok = mine && band_sample_ray(v, r, s, vx, vy, vz, dsq[0]);
+        float dsq = 0.0f;
+        const bool ok = mine && band_sample_ray(v, r, s, vx, vy, vz, dsq);
         // A straight ray leaves a block (a convex box) for good, so equal
         // consecutive blocks are the only repeats.
         const bool fresh = ok && (!started || (((vx ^ ox) | (vy ^ oy) | (vz ^ oz)) >> 3) != 0);
@@ -567,12 +559,12 @@ __device__ __forceinline__ void band_point(const DevVolume& v, const BatchArgs& 
         }
         resolve_grouped<MODE>(v, rest, (long long)k, res, hist, n_bins);
         if (RECORDS) tag_touched<true>(v, u, fresh && res.bi >= 0 && (rest || old), res.bi, res.slot);
-        uint32_t vox[1] = {kNoVoxel};
+        uint32_t vox = kNoVoxel;
         if (ok && res.bi >= 0)
-            vox[0] = (uint32_t)res.bi * kBlockVoxels + (uint32_t)(((vz & 7) * kBlockDim + (vy & 7)) * kBlockDim + (vx & 7));
+            vox = (uint32_t)res.bi * kBlockVoxels + (uint32_t)(((vz & 7) * kBlockDim + (vy & 7)) * kBlockDim + (vx & 7));
         if (counts_drops && ok && res.bi < 0) ++drops;
         if (RECORDS)
-            count_samples<S>(v, u, mine || (round == 0 && in_batch && !live), (uint32_t)a.n, r.dist, vox, dsq, 1, slot, counted,
+            count_samples<S, 1>(v, u, mine || (round == 0 && in_batch && !live), (uint32_t)a.n, r.dist, &vox, &dsq, 1, slot, counted,
                              [&](int) { return oracle_fix(v, a, r, vx, vy, vz); });
     }
 }
@@ -688,7 +680,7 @@ band_kernel(DevVolume v, BatchArgs a, UpdateScratch u, unsigned long long* hist,
 // Integrate (allocate + count-and-sum) of a batch of several frames: the
 // single-frame walk with each point's camera taken from the frame table.
 template <int S>
-__global__ void __launch_bounds__(kBandThreads, kBandMinBlocks)
+__global__ void __launch_bounds__(kBandThreads, kBandFramesMinBlocks)
 band_frames_kernel(DevVolume v, BatchArgs a, UpdateScratch u, const __grid_constant__ FrameTable frames) {
     grid_dependency_wait();
     band_tiles<kAllocInsert, true, S, true>(v, a, u, nullptr, 0, BatchPoints<0>{a}, FrameCursor(frames));
@@ -697,7 +689,7 @@ band_frames_kernel(DevVolume v, BatchArgs a, UpdateScratch u, const __grid_const
 // The same for several depth images of equal size: each CTA stages the
 // images' poses in shared memory first.
 template <int S>
-__global__ void __launch_bounds__(kBandThreads, kBandMinBlocks)
+__global__ void __launch_bounds__(kBandThreads, kBandFramesMinBlocks)
 band_depth_frames_kernel(DevVolume v, BatchArgs a, UpdateScratch u, const __grid_constant__ FrameTable frames,
                          const __grid_constant__ PoseTable poses) {
     __shared__ FramePose s_pose[kMaxDepthFrames];
@@ -740,7 +732,7 @@ __device__ __forceinline__ int scene_of(const int* begin, int n, int item) {
 // item's scene descriptor in shared memory and flushes its per-scene
 // counters whenever it moves to another scene.
 template <int S>
-__global__ void __launch_bounds__(kBandThreads, kBandMinBlocks)
+__global__ void __launch_bounds__(kBandThreads, kBandFramesMinBlocks)
 band_multi_kernel(StepWork w) {
     __shared__ BandSmem<false> sm;
     __shared__ SceneWork sw;
