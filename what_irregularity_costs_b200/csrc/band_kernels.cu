@@ -67,6 +67,12 @@ constexpr int kChunk = OSN_BAND_CHUNK;  // samples per ray walked together (9: t
 #ifndef OSN_BAND_FRAMES_MIN_BLOCKS
 #define OSN_BAND_FRAMES_MIN_BLOCKS 7
 #endif
+// Several depth images per call: the double-precision unprojection needs more
+// (four images 137.9 us at 7, 129.5 at 8, 125.7 at 6; one image is best at 8).
+#ifndef OSN_BAND_DEPTH_MIN_BLOCKS
+#define OSN_BAND_DEPTH_MIN_BLOCKS 6
+#endif
+constexpr int kBandDepthMinBlocks = OSN_BAND_DEPTH_MIN_BLOCKS;
 constexpr int kBandMinBlocks = OSN_BAND_MIN_BLOCKS;
 constexpr int kBandFramesMinBlocks = OSN_BAND_FRAMES_MIN_BLOCKS;
 
@@ -689,7 +695,7 @@ band_frames_kernel(DevVolume v, BatchArgs a, UpdateScratch u, const __grid_const
 // The same for several depth images of equal size: each CTA stages the
 // images' poses in shared memory first.
 template <int S>
-__global__ void __launch_bounds__(kBandThreads, kBandFramesMinBlocks)
+__global__ void __launch_bounds__(kBandThreads, kBandDepthMinBlocks)
 band_depth_frames_kernel(DevVolume v, BatchArgs a, UpdateScratch u, const __grid_constant__ FrameTable frames,
                          const __grid_constant__ PoseTable poses) {
     __shared__ FramePose s_pose[kMaxDepthFrames];
