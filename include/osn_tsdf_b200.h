@@ -32,7 +32,8 @@ typedef struct OsnTsdfCudaVolume OsnTsdfCudaVolume;
 /* Device pointers and parameters describing a volume's storage.
  * Same 104-byte layout as the reference (c_api.h:61-78, size asserted at
  * cpp/src/c_api_cuda.cu:14): table slots are (int64 key, int32 block_idx,
- * int32 pad); tsdf/weight/r/g/b hold weighted SUMS, 512 floats per block at
+ * int32 pad), the pad holding the number of the last update that touched the
+ * block; tsdf/weight/r/g/b hold weighted SUMS, 512 floats per block at
  * block_idx * 512, voxel (lx,ly,lz) at (lz*8+ly)*8+lx. */
 typedef struct {
     void* table;          /* hash_mask+1 live slots, then 2^20 scratch slots (key -2) */
@@ -411,12 +412,13 @@ int32_t osn_tsdf_batch_synchronize(OsnTsdfBatch* b);
  * with the same scenes and shape). */
 int32_t osn_tsdf_batch_set_graph(OsnTsdfBatch* b, int32_t enabled);
 /* Run the next 16 * steps_per_shape steps with each candidate shape
- * (band tiles per work item 1/2/4/8, warp-grouped or per-lane block
- * resolution, one or two blocks per finish item), then keep the fastest
- * median. Shapes change speed only, never results. */
+ * (band tiles per work item 1/2/4/8, each with every probe and finish_pair,
+ * which no longer change the passes), then keep the fastest median. Shapes
+ * change speed only, never results. */
 int32_t osn_tsdf_batch_autotune(OsnTsdfBatch* b, int32_t steps_per_shape);
 /* Fix the shape: tiles_per_item in [1, 8], probe 0 (warp) or 1 (lane),
- * finish_pair 0 or 1. */
+ * finish_pair 0 or 1. The last two are checked and reported back only: the
+ * walk has one way to resolve blocks and finish deals them out evenly. */
 int32_t osn_tsdf_batch_set_shape(OsnTsdfBatch* b, int32_t tiles_per_item, int32_t probe,
                                  int32_t finish_pair);
 /* Current shape into out3 (tiles_per_item, probe, finish_pair); returns 1

@@ -445,6 +445,7 @@ int32_t Volume::extract(float* posnor, uint8_t* rgb, int32_t cap, float min_w, f
     float* d_pos = posnor;
     uint8_t* d_rgb = rgb;
     if (host_out) {
+        if (block_count() <= 0) return 0;  // before any buffer is grown
         if (!ensure_mesh(cap, rgb != nullptr)) return -1;
         d_pos = mesh_posnor_;
         d_rgb = rgb ? mesh_rgb_ : nullptr;
