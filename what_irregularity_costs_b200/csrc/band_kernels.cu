@@ -338,10 +338,12 @@ __device__ __forceinline__ uint32_t measure_point(const DevVolume& v, const Ray&
 
 // Limits of the fast walk, in voxels. Coordinates below kReach: the floor is
 // exact and block coordinates fit a key. Below kSureReach, rounding errors
-// are small against a voxel, which the occlusion shortcut assumes. Samples
+// are small against a voxel, and beyond kSureDist from the camera the samples
+// behind it are not occluded either: the occlusion shortcut needs both. Samples
 // within kSpreadXY / kSpreadZ of the warp's first point: their offsets fit.
 constexpr float kReach = 2097152.0f;
 constexpr float kSureReach = 32768.0f;
+constexpr float kSureDist = 2.0f;
 constexpr float kSpreadXY = 1000.0f;
 constexpr float kSpreadZ = 490.0f;
 constexpr float kFloorMagic = 12582912.0f;  // 1.5 * 2^23
@@ -386,9 +388,12 @@ __device__ __forceinline__ uint32_t voxel_high(uint32_t w) {
 // 1.5 * 2^23 with rounding toward -infinity (exact for |x| < 2^22; the low
 // bits are then the voxel coordinate), and (vf + 0.5) * size is the single
 // fused rounding of vf * size + size / 2 (vf + 0.5 is exact). Within
-// kSureReach, a sample up to step trunc / voxel - 1 (v.sure_step) cannot be
-// occluded: its voxel's centre lies within 0.87 voxels of it and rounding
-// errors stay below 0.1 voxels.
+// kSureReach and beyond kSureDist, a sample up to step trunc / voxel - 1
+// (v.sure_step) cannot be occluded. Its voxel's centre lies within 0.87 voxels
+// of it and rounding errors stay below 0.1 voxels, so in front of the camera
+// sdf > -(s + 0.97) voxels. A sample behind the camera (s < 0, the point closer
+// than |s| voxels) has sdf > 2 dist - (|s| + 0.97) voxels, and |s| is less than
+// trunc / voxel + 1: above -trunc from a distance of 0.99 voxels on.
 //
 // FRAMES: the batch holds several frames; (cx, cy, cz) is the camera of
 // point i's frame (otherwise the batch's one camera is used).
@@ -435,7 +440,8 @@ __device__ __forceinline__ void band_point(const DevVolume& v, const BatchArgs& 
         const unsigned group = __ballot_sync(0xffffffffu, mine);
         if (todo != 0u && (group == 0u || round == 3)) break;  // warp-uniform
         // Steps up to this one need no occlusion test.
-        const int sure_step = __all_sync(0xffffffffu, far < kSureReach || !mine) ? v.sure_step : INT_MIN;
+        const bool sure = far < kSureReach && r.dist >= kSureDist * v.voxel_size;
+        const int sure_step = __all_sync(0xffffffffu, sure || !mine) ? v.sure_step : INT_MIN;
         const bool writes = mine || (round == 0 && in_batch && !live);
         uint32_t slot = (uint32_t)i;  // band slot (s = -steps, i)
         // The warp's origin as raw floor bits.
