@@ -503,6 +503,7 @@ SceneWork Volume::batch_work(const BatchArgs& a, cudaStream_t s) {
     w.u = us_;
     w.u.tag = update_tag_;
     ctl_clear_ = false;  // the step uses the first control block
+    if (a.n > 0) last_ctl_ = us_.ctl;  // an idle scene keeps its last update's counters
     w.band_tiles = (a.n + kBatchTilePoints - 1) / kBatchTilePoints;
     w.n_slots = (int32_t)batch_records(a.n, dv_.steps);
     return w;
