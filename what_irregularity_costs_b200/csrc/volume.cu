@@ -335,6 +335,12 @@ cudaError_t Volume::run_update(const BatchArgs& a, const UpdateScratch& scratch,
     // final weights, so a stale read only lets through a sample finish rejects.
     const bool pipe = pipelined_ && scratch.ctl == us_.ctl;  // not the fixed no-alloc scratch
     if (pipelined_ && !pipe) join();
+    // An update recorded by a stream capture does not run now, and may run any
+    // number of times later, always with the same update number: from here on
+    // no update of this volume may rely on what another one cleared.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (!captured_ && cudaStreamIsCapturing(stream_, &capture) == cudaSuccess && capture != cudaStreamCaptureStatusNone)
+        captured_ = true;
     // Block tags are update numbers; at the (theoretical) wrap, clear them.
     if (++update_tag_ == 0u) {
         join();
@@ -358,7 +364,7 @@ cudaError_t Volume::run_update(const BatchArgs& a, const UpdateScratch& scratch,
     cudaError_t e = cudaSuccess;
     if (pipe) e = cudaStreamWaitEvent(stream_, tail_done_[p], 0);
     bool clear = true;
-    if (!pipelined_ && scratch.ctl == us_.ctl) {
+    if (!pipelined_ && !captured_ && scratch.ctl == us_.ctl) {
         u.ctl = us_.ctl + ctl_turn_;
         u.next_ctl = us_.ctl + (ctl_turn_ ^ 1);
         clear = !ctl_clear_;
@@ -518,10 +524,10 @@ cudaError_t Volume::reset() {
     mark_end(kKReset);
     if (e == cudaSuccess) e = cudaMemsetAsync(counters_, 0, sizeof(VolumeCounters), stream_);
     // Every completed update leaves the per-voxel batch state at zero, so it is
-    // cleared here only when an update stopped on an error half way (the 12
-    // bytes per voxel of a 2^19-block pool took 0.52 ms, ten times the rest of
-    // a reset).
-    if (e == cudaSuccess && unfinished_) {
+    // cleared here only when an update stopped on an error half way or was
+    // captured (the 12 bytes per voxel of a 2^19-block pool took 0.52 ms, ten
+    // times the rest of a reset).
+    if (e == cudaSuccess && (unfinished_ || captured_)) {
         const size_t n_vox = (size_t)dv_.pool_capacity * kBlockVoxels;
         e = cudaMemsetAsync(us_.vcnt, 0, n_vox * sizeof(uint32_t), stream_);
         if (e == cudaSuccess) e = cudaMemsetAsync(us_.vacc, 0, n_vox * sizeof(unsigned long long), stream_);

@@ -30,7 +30,8 @@ enum KernelId : int {
 // Counters an update keeps on the device, zero when it starts. Serial updates
 // take two control blocks in turn: each update's finish pass clears the other
 // one for the next (a memset of its own before every walk cost 2-3 us a call).
-// Pipelined, batched and no-alloc updates clear theirs first.
+// Pipelined, batched and no-alloc updates clear theirs first, and so do all
+// updates of a volume of which one was recorded by a stream capture.
 struct UpdateControl {
     int32_t n_records;   // band records counted (contributions that can be accepted)
     int32_t n_touched;   // blocks that received a band sample
@@ -238,6 +239,8 @@ private:
     // An update that did not queue all of its passes may have left per-voxel
     // batch state behind: the next reset clears all of it.
     bool unfinished_ = false;
+    // A stream capture recorded an update of this volume.
+    bool captured_ = false;
     float weight_cap_ = 0.0f;
     cudaStream_t stream_ = nullptr;
     UpdateScratch us_{};
