@@ -256,7 +256,7 @@ __device__ __forceinline__ void count_samples(const DevVolume& v, const UpdateSc
     if (capped) {
         float w0[N];
 #pragma unroll
-        for (int j = 0; j < N; ++j) w0[j] = weight_at<S>(v, at[j] == kNoVoxel ? 0u : at[j]);
+        for (int j = 0; j < N; ++j) w0[j] = weight_in_update<S>(v.weight, at[j] == kNoVoxel ? 0u : at[j]);
 #pragma unroll
         for (int j = 0; j < N; ++j)
             if (w0[j] >= v.weight_cap) at[j] = kNoVoxel;  // takes no contribution

@@ -482,15 +482,6 @@ __device__ __forceinline__ void finish_voxel(const SelectArgs& v, uint32_t vi, i
     v.vcnt[vi] = 0u;
 }
 
-// The weight of voxel vi before the batch (finish leaves crossing voxels as they were).
-template <int S>
-__device__ __forceinline__ float weight_before(const SelectArgs& v, uint32_t vi) {
-    if constexpr (S == kStoreF16U16)
-        return (float)__ldg(reinterpret_cast<const unsigned short*>(v.weight) + vi);
-    else
-        return __ldg(v.weight + vi);
-}
-
 // Sum of the accepted values of a group of at most 32 * R records, by one
 // warp: record r * 32 + lane in registers, ranked by id against every other
 // record with shuffles; a record is accepted when fewer than keep ids are
@@ -608,7 +599,8 @@ __device__ __forceinline__ int select_group(const SelectArgs& sa, const DevVolum
     const unsigned long long h = __ldcg(&sa.vacc[vi]);
     const uint32_t base = (uint32_t)(h >> 32) - 1u;
     const int n = (int)(uint32_t)h;
-    const int keep = accept_count(weight_before<S>(sa, vi), sa.cap, n);
+    // The weight before the batch: finish leaves crossing voxels as they were.
+    const int keep = accept_count(weight_in_update<S>(sa.weight, vi), sa.cap, n);
     long long fix = 0ll;
     if ((uint64_t)base + (uint64_t)n > (uint64_t)sa.record_cap) {
         // Counters left by a failed update: nothing to rank.
@@ -648,7 +640,7 @@ __device__ __forceinline__ uint32_t crossing_slots(const UpdateScratch& u, const
 #pragma unroll
     for (int m = 0; m < kGroupPerThread; ++m) {
         same[m] = m > 0 && vi[m] != kNoVoxel && vi[m - 1] != kNoVoxel && (vi[m - 1] >> 5) == (vi[m] >> 5);
-        word[m] = (vi[m] == kNoVoxel || same[m]) ? 0u : __ldg(&u.xbits[vi[m] >> 5]);
+        word[m] = (vi[m] == kNoVoxel || same[m]) ? 0u : __ldca(&u.xbits[vi[m] >> 5]);
     }
     uint32_t cross = 0u;
 #pragma unroll

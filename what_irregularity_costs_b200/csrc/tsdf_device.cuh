@@ -112,14 +112,25 @@ __host__ __device__ constexpr int tsdf_bytes(int storage) {
 }
 __host__ __device__ constexpr int weight_bytes(int storage) { return storage == kStoreF16U16 ? 2 : 4; }
 
-// Weight of voxel i (read-only path: kernels that run after the volume's
-// weights were last written).
+// Weight of voxel i. Read-only path: for kernels that are launched after the
+// volume's weights were last written, none of whose life overlaps an update (a
+// non-coherent load wants data that nothing writes while the kernel lives).
 template <int S>
 __device__ __forceinline__ float weight_at(const DevVolume& v, size_t i) {
     if constexpr (S == kStoreF16U16)
         return (float)__ldg(reinterpret_cast<const unsigned short*>(v.weight) + i);
     else
         return __ldg(v.weight + i);
+}
+
+// The same for the passes of an update, whose CTAs may be launched while the
+// pass that writes the weights still runs (they wait for it before they read).
+template <int S>
+__device__ __forceinline__ float weight_in_update(const float* weight, size_t i) {
+    if constexpr (S == kStoreF16U16)
+        return (float)__ldca(reinterpret_cast<const unsigned short*>(weight) + i);
+    else
+        return __ldca(weight + i);
 }
 
 // Mean normalised TSDF of voxel i given its weight w (sum * (1/w) for FP32
