@@ -411,10 +411,9 @@ int32_t osn_tsdf_batch_synchronize(OsnTsdfBatch* b);
 /* Replay the step's passes from a CUDA graph (captured on the second step
  * with the same scenes and shape). */
 int32_t osn_tsdf_batch_set_graph(OsnTsdfBatch* b, int32_t enabled);
-/* Run the next 16 * steps_per_shape steps with each candidate shape
- * (band tiles per work item 1/2/4/8, each with every probe and finish_pair,
- * which no longer change the passes), then keep the fastest median. Shapes
- * change speed only, never results. */
+/* Run the next 4 * steps_per_shape steps with each candidate shape (band
+ * tiles per work item 1/2/4/8), then keep the fastest median. Shapes change
+ * speed only, never results. */
 int32_t osn_tsdf_batch_autotune(OsnTsdfBatch* b, int32_t steps_per_shape);
 /* Fix the shape: tiles_per_item in [1, 8], probe 0 (warp) or 1 (lane),
  * finish_pair 0 or 1. The last two are checked and reported back only: the

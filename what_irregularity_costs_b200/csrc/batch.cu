@@ -17,9 +17,9 @@
 // The passes after the upload are launched with programmatic stream
 // serialisation and can be captured once into a CUDA graph and replayed
 // every step (their arguments only point at the table). An autotuner runs
-// the next steps with each candidate shape (tiles per band item, block
-// resolution scheme, blocks per finish item) and keeps the fastest; every
-// shape computes bit-identical results, so tuning uses live steps.
+// the next steps with each candidate shape (tiles per band item) and keeps the
+// fastest; every shape computes bit-identical results, so tuning uses live
+// steps.
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
@@ -221,15 +221,11 @@ public:
     // keep the one with the smallest median step time.
     void autotune(int steps_per_shape) {
         candidates_.clear();
-        for (int tiles : {1, 2, 4, 8})
-            for (int probe : {0, 1})
-                for (int pair : {1, 0}) {
-                    BatchShape s;
-                    s.band_tiles_per_item = tiles;
-                    s.probe = probe;
-                    s.finish_pair = pair;
-                    candidates_.push_back(s);
-                }
+        for (int tiles : {1, 2, 4, 8}) {
+            BatchShape s;
+            s.band_tiles_per_item = tiles;
+            candidates_.push_back(s);
+        }
         steps_per_shape_ = std::max(1, steps_per_shape);
         tune_index_ = 0;
         tune_step_ = 0;
@@ -260,9 +256,9 @@ private:
         cudaEvent_t start, end;
     };
 
+    // The passes are the same (probe and finish_pair do not reach them).
     static bool same(const BatchShape& a, const BatchShape& b) {
-        return a.band_tiles_per_item == b.band_tiles_per_item && a.probe == b.probe &&
-               a.finish_pair == b.finish_pair;
+        return a.band_tiles_per_item == b.band_tiles_per_item;
     }
 
     StepWork work(int n, const BatchShape& shape) const {
@@ -463,15 +459,16 @@ int32_t osn_tsdf_batch_shape(OsnTsdfBatch* b, int32_t* out3) {
 int32_t osn_tsdf_batch_tune_results(OsnTsdfBatch* b, double* ms, int32_t* shapes, int32_t n_max) {
     osn_b200::Batch* x = batch_of(b);
     if (!x || n_max <= 0) return 0;
+    // Every candidate with each probe and finish_pair, which have its time.
     const std::vector<double> med = x->tune_results();
     const auto& cand = x->candidates();
-    const int n = std::min<int>((int)med.size(), n_max);
+    const int n = std::min<int>(4 * (int)med.size(), n_max);
     for (int k = 0; k < n; ++k) {
-        if (ms) ms[k] = med[k];
+        if (ms) ms[k] = med[k / 4];
         if (shapes) {
-            shapes[3 * k + 0] = cand[k].band_tiles_per_item;
-            shapes[3 * k + 1] = cand[k].probe;
-            shapes[3 * k + 2] = cand[k].finish_pair;
+            shapes[3 * k + 0] = cand[k / 4].band_tiles_per_item;
+            shapes[3 * k + 1] = (k >> 1) & 1;
+            shapes[3 * k + 2] = 1 - (k & 1);
         }
     }
     return n;

@@ -326,7 +326,7 @@ class Server:
                         s.stage_ev[buf] = ev
                     inflight.append((ev, members))
                     self.steps += 1
-                    if self.steps == 16 * max(self.autotune_steps, 0):
+                    if self.steps == 4 * max(self.autotune_steps, 0):
                         self.t_tuned = time.perf_counter() - t0
                     continue
             if inflight:
