@@ -64,8 +64,8 @@ Volume::Volume(float voxel, int32_t pool, float trunc_m, float weight_cap, uint3
     weight_cap_ = weight_cap;
     dv_.pool_capacity = pool;
     dv_.steps = std::max(1, (int32_t)std::ceil(dv_.trunc * dv_.inv_voxel));
-    dv_.sure_step = -dv_.steps - 1;
-    while (dv_.sure_step < dv_.steps && (float)(dv_.sure_step + 2) * voxel <= dv_.trunc) ++dv_.sure_step;
+    dv_.sure_step = dv_.steps;  // at most two above the answer, whatever the band's length
+    while (dv_.sure_step >= -dv_.steps && !((float)(dv_.sure_step + 1) * voxel <= dv_.trunc)) --dv_.sure_step;
     dv_.spin_limit = kSpinLimit;
     ok_ = alloc_device(hash_slots);
 }
