@@ -25,10 +25,11 @@ def directions(n, rmin, rmax, seed):
 
 
 def line(axis):
-    """Warps whose points step from their first by 4.4 to 5.0 m on one axis:
-    the spread of a warp's table (480 voxels, the band included) lies between."""
+    """Warps whose points step from their first by 9.4 to 10 m in x or y, 4.4 to
+    5 m in z: the spread of a warp's table (990 and 480 voxels, the band
+    included) lies between."""
     p = np.tile(np.array([[1.0, 1.1, 1.2]]), (640, 1)) + 0.03 * directions(640, 0.1, 1.0, 3)
-    p[:, axis] += np.where(np.arange(640) % 32 == 0, 0.0, 4.4 + 0.6 * (np.arange(640) % 32) / 31.0)
+    p[:, axis] += np.where(np.arange(640) % 32 == 0, 0.0, (4.4 if axis == 2 else 9.4) + 0.6 * (np.arange(640) % 32) / 31.0)
     return p.astype(np.float32)
 
 

@@ -20,7 +20,7 @@
 //
 // What bounds it (four 640x480 frames a call): L1 throughput of the scattered
 // weight gathers and reductions (about 21 M sectors, one a cycle per SM: 75
-// us) and instruction issue (53 M warp instructions: 48 us); 104 us measured.
+// us) and instruction issue (57 M warp instructions: 50 us); 104 us measured.
 // 143 before the table (67 M instructions, and values spilled around calls);
 // 121 with the samples in registers, whose columns left room for fewer loads in
 // flight than shared memory does.
@@ -345,24 +345,26 @@ __device__ __forceinline__ uint32_t measure_point(const DevVolume& v, const Ray&
 // exact and block coordinates fit a key. Below kSureReach, rounding errors
 // are small against a voxel, and beyond kSureDist from the camera the samples
 // behind it are not occluded either: the occlusion shortcut needs both. Samples
-// within kSpread of the warp's first point share its table: as far as offsets of
-// 10 bits reach, since pixels on both sides of a depth edge still share blocks
-// (at 128, the walk of a mapped 640x480 room took 10 % longer; shuffled clouds
-// were the same to 2 %).
+// within kSpreadXY and kSpreadZ of the warp's first point share its table: as far
+// as offsets of 11 and 10 bits reach, since pixels on both sides of a depth edge
+// still share blocks (at 128, the walk of a mapped 640x480 room took 10 % longer;
+// at 480, a band of 100 voxels 137 us instead of 84; shuffled clouds were the same
+// to 2 %).
 constexpr float kReach = 4194000.0f;  // 2^22 and rounding
 constexpr float kSureReach = 32768.0f;
 constexpr float kSureDist = 2.0f;
-constexpr float kSpread = 480.0f;
+constexpr float kSpreadXY = 990.0f;
+constexpr float kSpreadZ = 480.0f;
 constexpr float kFloorMagic = 12582912.0f;  // 1.5 * 2^23
 constexpr uint32_t kFloorBits = 0x4B400000u;  // its bits
 constexpr uint32_t kNoOffset = 0xFFFFFFFFu;  // no sample; no block
-constexpr uint32_t kOriginBack = 512u;       // voxels from the origin to its point's block
+constexpr uint32_t kBackXY = 1024u, kBackZ = 512u;  // voxels from the origin to its point's block
 static_assert(kNoOffset == kNoVoxel, "a sample's column holds its offset, then its voxel");
-static_assert(kSpread + 16.0f < (float)kOriginBack, "offsets of 10 bits");
+static_assert(kSpreadXY + 16.0f < (float)kBackXY && kSpreadZ + 16.0f < (float)kBackZ, "offsets of 11 and 10 bits");
 
-// Raw floor bits of the origin kOriginBack voxels before the block at x.
-__device__ __forceinline__ uint32_t origin_bits(float x, float inv_voxel) {
-    return (__float_as_uint(__fadd_rd(__fmul_rn(x, inv_voxel), kFloorMagic)) & ~7u) - kOriginBack;
+// Raw floor bits of the origin `back` voxels before the block at x.
+__device__ __forceinline__ uint32_t origin_bits(float x, float inv_voxel, uint32_t back) {
+    return (__float_as_uint(__fadd_rd(__fmul_rn(x, inv_voxel), kFloorMagic)) & ~7u) - back;
 }
 // A voxel's offset from an origin: x (11 bits), y << 11 (11 bits), z << 22 (10
 // bits). An offset without the low three bits of its fields is its block's key
@@ -559,13 +561,14 @@ __device__ __forceinline__ void band_point(const DevVolume& v, const BatchArgs& 
     const int first = fit ? __ffs(fit) - 1 : 0;
     const float fx = __shfl_sync(0xffffffffu, px, first), fy = __shfl_sync(0xffffffffu, py, first),
                 fz = __shfl_sync(0xffffffffu, pz, first);
-    const bool tabled = fits && v.inv_voxel * fmaxf(fmaxf(fabsf(px - fx), fabsf(py - fy)), fabsf(pz - fz)) +
-                                        band < kSpread;
+    const bool tabled = fits && v.inv_voxel * fmaxf(fabsf(px - fx), fabsf(py - fy)) + band < kSpreadXY &&
+                        v.inv_voxel * fabsf(pz - fz) + band < kSpreadZ;
     // Steps up to this one need no occlusion test.
     const bool sure = far < kSureReach && r.dist >= kSureDist * v.voxel_size;
     const int sure_step = __all_sync(0xffffffffu, sure || !fits) ? v.sure_step : INT_MIN;
     // The warp's origin as raw floor bits.
-    const uint32_t ox = origin_bits(fx, v.inv_voxel), oy = origin_bits(fy, v.inv_voxel), oz = origin_bits(fz, v.inv_voxel);
+    const uint32_t ox = origin_bits(fx, v.inv_voxel, kBackXY), oy = origin_bits(fy, v.inv_voxel, kBackXY),
+                   oz = origin_bits(fz, v.inv_voxel, kBackZ);
     uint32_t base = pack_offset(ox, oy, oz);
     uint32_t slot = (uint32_t)i;  // band slot (s = -steps, i)
     uint32_t* const vox = &sm.vox[0][threadIdx.x];  // voxel offset, then the voxel's index
@@ -578,9 +581,9 @@ __device__ __forceinline__ void band_point(const DevVolume& v, const BatchArgs& 
         __syncwarp();
         if (fits && !tabled) {  // this lane's origin: by the chunk's first sample
             const float t = __fmul_rn((float)c0, v.voxel_size);
-            base = pack_offset(origin_bits(__fadd_rn(px, __fmul_rn(r.ux, t)), v.inv_voxel),
-                               origin_bits(__fadd_rn(py, __fmul_rn(r.uy, t)), v.inv_voxel),
-                               origin_bits(__fadd_rn(pz, __fmul_rn(r.uz, t)), v.inv_voxel));
+            base = pack_offset(origin_bits(__fadd_rn(px, __fmul_rn(r.ux, t)), v.inv_voxel, kBackXY),
+                               origin_bits(__fadd_rn(py, __fmul_rn(r.uy, t)), v.inv_voxel, kBackXY),
+                               origin_bits(__fadd_rn(pz, __fmul_rn(r.uz, t)), v.inv_voxel, kBackZ));
         }
 #pragma unroll
         for (int j = 0; j < kChunk; ++j) {

@@ -434,9 +434,7 @@ __device__ __forceinline__ uint32_t entry_id(const DevVolume& v, const BatchArgs
         return (uint32_t)e;
 }
 
-// What the selection of one cap-crossing voxel touches, as plain values: an
-// out-of-line selection takes these, so no kernel parameter is passed by
-// address (which would make every thread copy it to local memory).
+// What the selection of a cap-crossing voxel touches, as plain values.
 struct SelectArgs {
     float* tsdf;
     float* weight;
@@ -950,8 +948,8 @@ finish_multi_kernel(StepWork w) {
     if (t < w.n_scenes && s_updated[t]) atomicAdd(&s_args[t].ctl->n_updated, s_updated[t]);
 }
 
-// Group, select and finish the cap-crossing voxels of every scene that has
-// any: work items of 2048 band slots of one scene.
+// Place the records of the cap-crossing voxels of every scene that has any:
+// work items of 2048 band slots of one scene.
 template <int S>
 __global__ void __launch_bounds__(kGroupThreads, OSN_GROUP_MIN_BLOCKS)
 group_multi_kernel(StepWork w) {
@@ -1059,8 +1057,7 @@ cudaError_t launch_finish(const DevVolume& v, const UpdateScratch& u, int sm_cou
     }
 }
 
-cudaError_t launch_group(const DevVolume& v, const BatchArgs& a, const UpdateScratch& u, int sm_count,
-                         cudaStream_t s) {
+cudaError_t launch_group(const DevVolume& v, const BatchArgs& a, const UpdateScratch& u, cudaStream_t s) {
     const uint32_t n_slots = (uint32_t)a.n * (2u * (uint32_t)v.steps + 1u);
     if (n_slots == 0) return cudaSuccess;
     const uint32_t per_cta = kGroupThreads * (uint32_t)kGroupPerThread;

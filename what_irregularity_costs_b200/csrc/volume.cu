@@ -389,7 +389,7 @@ cudaError_t Volume::run_update(const BatchArgs& a, const UpdateScratch& scratch,
     if (e != cudaSuccess) return e;
     if (dv_.weight_cap > 0.0f) {  // without a cap no voxel crosses it
         mark_start(kKGroup, tail);
-        e = launch_group(dv_, a, u, sm_count_, tail);
+        e = launch_group(dv_, a, u, tail);
         mark_end(kKGroup, tail);
         if (e != cudaSuccess) return e;
         mark_start(kKSelect, tail);

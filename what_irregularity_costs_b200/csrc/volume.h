@@ -18,9 +18,8 @@ enum KernelId : int {
     kKAllocate = 0,      // allocate-only band walk
     kKBand = 1,          // count-and-sum band walk (fused with allocation in integrate)
     kKFinish = 2,        // per touched block: finish every voxel that accepts all its records
-    kKGroup = 3,         // records of voxels that cross the cap: grouped per voxel, ordered
-                         // cap selection, voxel finished
-    kKSelect = 4,        // ordered cap selection of the crossing voxels (its own pass)
+    kKGroup = 3,         // records of voxels that cross the cap, grouped per voxel
+    kKSelect = 4,        // ordered cap selection of the crossing voxels, voxels finished
     kKExtract = 5,
     kKReset = 6,
     kKUnused7 = 7,       // no longer launched
@@ -325,8 +324,8 @@ cudaError_t launch_list_blocks(const DevVolume& v, int32_t* out, int32_t* count,
 cudaError_t launch_extract(const DevVolume& v, const int32_t* list, const int32_t* count, float min_w, float iso,
                            float* posnor, uint8_t* rgb, int32_t cap, int32_t* ctl, int sm_count, cudaStream_t s);
 
-// The update pipeline: band walk (counts, sums, records) -> finish -> group
-// (grouping, ordered selection and finishing of the voxels that cross the cap).
+// The update pipeline: band walk (counts, sums, records) -> finish -> group ->
+// select (the last two for the voxels that cross the cap).
 cudaError_t launch_band_records(const DevVolume& v, const BatchArgs& a, const UpdateScratch& u,
                                 bool insert, int sm_count, cudaStream_t s);
 // Several-frame integrate: the walk with per-frame cameras (FP32 / FP16 storage).
@@ -337,8 +336,7 @@ cudaError_t launch_band_frames(const DevVolume& v, const BatchArgs& a, const Upd
 cudaError_t launch_band_depth_frames(const DevVolume& v, const BatchArgs& a, const UpdateScratch& u,
                                      const FrameTable& frames, const PoseTable& poses, int sm_count, cudaStream_t s);
 cudaError_t launch_finish(const DevVolume& v, const UpdateScratch& u, int sm_count, cudaStream_t s);
-cudaError_t launch_group(const DevVolume& v, const BatchArgs& a, const UpdateScratch& u, int sm_count,
-                         cudaStream_t s);
+cudaError_t launch_group(const DevVolume& v, const BatchArgs& a, const UpdateScratch& u, cudaStream_t s);
 cudaError_t launch_select(const DevVolume& v, const BatchArgs& a, const UpdateScratch& u, int sm_count,
                           cudaStream_t s);
 
