@@ -201,8 +201,7 @@ int64_t Volume::evict_chunks(int32_t lo, int32_t hi, void* host, int64_t cap) {
               cudaMemcpyAsync(d_order, order.data(), (size_t)b * sizeof(int32_t), cudaMemcpyHostToDevice,
                               stream_) == cudaSuccess;
     if (ok) {
-        gather_blocks_kernel<<<b, kCopyThreads, 0, stream_>>>(pool, stage, d_order, b);
-        ok = cudaGetLastError() == cudaSuccess;
+        ok = launch_now(gather_blocks_kernel, b, kCopyThreads, stream_, pool, stage, d_order, b) == cudaSuccess;
     }
     // The blocks that stay, back to the front of the pool.
     ok = ok && cudaMemcpyAsync(pool.coord, stage.coord, (size_t)n_keep * sizeof(BlockCoord),
@@ -272,8 +271,7 @@ int32_t Volume::stream_in(const void* host, int64_t size, int32_t* skipped) {
         p += bytes;
     }
     if (ok) {
-        stream_in_kernel<<<n, kCopyThreads, 0, stream_>>>(dv_, pool, pack, n, d_counts);
-        ok = cudaGetLastError() == cudaSuccess;
+        ok = launch_now(stream_in_kernel, n, kCopyThreads, stream_, dv_, pool, pack, n, d_counts) == cudaSuccess;
     }
     int32_t* hs = reinterpret_cast<int32_t*>(host_small_);
     ok = ok && cudaMemcpyAsync(hs, d_counts, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, stream_) == cudaSuccess &&

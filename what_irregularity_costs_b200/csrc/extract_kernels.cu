@@ -567,8 +567,8 @@ static cudaError_t launch_extract_as(const DevVolume& v, const int32_t* list, co
             per_sm < 1)
             per_sm = 1;
     });
-    extract_kernel<S, COL><<<per_sm * sm_count, kExtractThreads, 0, s>>>(v, list, count, min_w, iso, posnor, rgb, cap, ctl);
-    return cudaGetLastError();
+    return launch_now(extract_kernel<S, COL>, per_sm * sm_count, kExtractThreads, s, v, list, count, min_w, iso, posnor,
+                      rgb, cap, ctl);
 }
 
 cudaError_t launch_extract(const DevVolume& v, const int32_t* list, const int32_t* count, float min_w, float iso,
@@ -592,26 +592,23 @@ cudaError_t launch_extract(const DevVolume& v, const int32_t* list, const int32_
 cudaError_t launch_reset_table(HashEntry* first, uint32_t count, long long key, cudaStream_t s) {
     if (count == 0) return cudaSuccess;
     const int grid = (int)std::min<uint32_t>((count + 255) / 256, 148u * 16u);
-    reset_table_kernel<<<grid, 256, 0, s>>>(first, count, key);
-    return cudaGetLastError();
+    return launch_now(reset_table_kernel, grid, 256, s, first, count, key);
 }
 
 cudaError_t launch_list_blocks(const DevVolume& v, int32_t* out, int32_t* count, cudaStream_t s) {
     const uint32_t size = v.hash_mask + 1;
     const int grid = (int)std::min<uint32_t>((size + 255) / 256, 148u * 8u);
-    list_blocks_kernel<<<grid, 256, 0, s>>>(v.table, size, out, count);
-    return cudaGetLastError();
+    return launch_now(list_blocks_kernel, grid, 256, s, v.table, size, out, count);
 }
 
 cudaError_t launch_reset(const DevVolume& v, const int32_t* list, const int32_t* count, cudaStream_t s) {
     // One wave of 16 CTAs per SM, striding over the blocks and the slots.
     const int grid = 148 * 16;
     switch (v.storage) {
-        case kStoreF16U16: reset_kernel<kStoreF16U16><<<grid, kResetThreads, 0, s>>>(v, list, count); break;
-        case kStoreF64: reset_kernel<kStoreF64><<<grid, kResetThreads, 0, s>>>(v, list, count); break;
-        default: reset_kernel<kStoreF32><<<grid, kResetThreads, 0, s>>>(v, list, count);
+        case kStoreF16U16: return launch_now(reset_kernel<kStoreF16U16>, grid, kResetThreads, s, v, list, count);
+        case kStoreF64: return launch_now(reset_kernel<kStoreF64>, grid, kResetThreads, s, v, list, count);
+        default: return launch_now(reset_kernel<kStoreF32>, grid, kResetThreads, s, v, list, count);
     }
-    return cudaGetLastError();
 }
 
 }  // namespace osn_b200

@@ -21,6 +21,7 @@
 #include <cstdio>
 
 #include "../../include/osn_tsdf_b200.h"
+#include "volume.h"
 
 namespace {
 
@@ -77,8 +78,7 @@ l2_probe_kernel(void* buf, unsigned long long n_words, int iters, unsigned* sink
 template <int KIND>
 cudaError_t run_probe(void* buf, unsigned long long n_words, int iters, int grid, unsigned* sink,
                       cudaStream_t s) {
-    l2_probe_kernel<KIND><<<grid, kProbeThreads, 0, s>>>(buf, n_words, iters, sink);
-    return cudaGetLastError();
+    return osn_b200::launch_now(l2_probe_kernel<KIND>, grid, kProbeThreads, s, buf, n_words, iters, sink);
 }
 
 cudaError_t launch_probe(int kind, void* buf, unsigned long long n_words, int iters, int grid, unsigned* sink,

@@ -73,8 +73,7 @@ size_t voxel_arrays(int storage, const DevVolume& d, void* out[5], size_t bytes[
 
 cudaError_t launch_rebuild_table(const DevVolume& v, int32_t n_blocks, cudaStream_t s) {
     if (n_blocks <= 0) return cudaSuccess;
-    rebuild_table_kernel<<<(n_blocks + 255) / 256, 256, 0, s>>>(v, n_blocks);
-    return cudaGetLastError();
+    return launch_now(rebuild_table_kernel, (n_blocks + 255) / 256, 256, s, v, n_blocks);
 }
 
 int64_t Volume::snapshot_bytes() {

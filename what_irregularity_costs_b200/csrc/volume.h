@@ -285,6 +285,19 @@ private:
     int64_t acc_launches_[kNumKernelIds] = {};
 };
 
+// Launch `kernel`; returns what this launch returned. (The runtime's last error
+// may be an earlier call's, such as an allocation that failed: a reset that took
+// it for its own stopped half way.)
+template <typename... KArgs, typename... Args>
+cudaError_t launch_now(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t s, Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = 0;
+    cfg.stream = s;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
 // Launch `kernel` with programmatic stream serialisation: it may begin while
 // the previous kernel on the stream is still running, and waits for it in
 // grid_dependency_wait().
