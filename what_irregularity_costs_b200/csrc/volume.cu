@@ -246,8 +246,6 @@ bool Volume::ensure_records(int64_t n_records) {
     if (cudaMalloc(&us_.grp, (size_t)n_records * sizeof(unsigned long long)) != cudaSuccess) return false;
     const int64_t n_cross = n_records / 2 + 1;  // a crossing voxel holds at least two records
     if (cudaMalloc(&us_.xlist, (size_t)n_cross * sizeof(uint32_t)) != cudaSuccess) return false;
-    us_.record_cap = n_records;
-    us_.xlist_cap = n_cross;
     if (pipelined_) {  // the second set's records and slot values grow with the first
         cudaFree(us2_.records);
         cudaFree(us2_.slot_val);
@@ -256,6 +254,9 @@ bool Volume::ensure_records(int64_t n_records) {
         if (cudaMalloc(&us2_.records, (size_t)n_records * sizeof(uint32_t)) != cudaSuccess) return false;
         if (cudaMalloc(&us2_.slot_val, (size_t)n_records * sizeof(float)) != cudaSuccess) return false;
     }
+    // Only with every buffer there: a call that fits would not look again.
+    us_.record_cap = n_records;
+    us_.xlist_cap = n_cross;
     return true;
 }
 
